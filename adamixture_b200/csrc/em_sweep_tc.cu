@@ -308,33 +308,55 @@ __global__ void q_to_tiles_kernel(const float* __restrict__ Q, int64_t N, int K,
 }
 
 // G tile (32 packed rows x 128 samples) into a shared-memory stage by the producer warp: lane
-// l copies row l. Whole 16-byte chunks go by cp.async and the lane's arrival on `bar` fires
-// when they land; rows that end past N, or a sample count that is not a multiple of 16,
-// take byte loads (0xFF, all missing, past the ends) and a plain arrival.
-__device__ __forceinline__ void producer_load_g(const Args& a, int64_t row0, int64_t i0, bool vec16,
-                                                uint8_t* gs, uint32_t bar) {
+// l copies row l as whole 16-byte chunks by cp.async, and the lane's arrival on `bar` fires
+// when they land. AL: every packed row starts 16-byte aligned (N % 16 == 0 and G aligned), 8
+// chunks. Otherwise the 9 chunks from the 16-byte boundary at or below the row's first byte
+// (they cover the 128 samples at any offset); the consumers apply the offset, which is a
+// constant of the row within the tile (row_offset). A sample count that is not a multiple of
+// 16 is what real cohorts have: loading such rows byte by byte through one warp took 14.9 ms
+// where these chunks take 2.7 ms (N=10,007 x M=200,003, K=8), the aligned shape's time.
+// Chunks that would leave the matrix (the last row or two) take byte loads; bytes past the
+// matrix are 0xFF (missing). Samples past N read the next row's bytes or 0xFF: their Q rows
+// are zero, so they add nothing to A and B, and their T is not written. Rows past the matrix
+// are not loaded: the consumers count them as missing.
+template <bool AL>
+__device__ __forceinline__ void producer_load_g(const Args& a, int64_t row0, int64_t i0, uint8_t* gs, uint32_t bar) {
+  constexpr int CHUNKS = AL ? TILE / 16 : TILE / 16 + 1;
+  static_assert(16 * CHUNKS <= G_ROW, "the chunks fit the padded row");
   const int l = threadIdx.x & 31;
   const int64_t row = row0 + l;
   const int64_t rows = (a.M + 3) >> 2;
   uint8_t* dst = gs + l * G_ROW;
-  if (row < rows && vec16 && i0 + TILE <= a.N) {
-    const uint8_t* src = a.G + row * a.N + i0;
+  if (row >= rows) {
+    mbar_arrive(bar);
+    return;
+  }
+  const uint8_t* src = a.G + row * a.N + i0;
+  if constexpr (!AL) src -= reinterpret_cast<uintptr_t>(src) & 15;
+  const uint8_t* end = a.G + rows * a.N;
+  if (src >= a.G && src + 16 * CHUNKS <= end) {
 #pragma unroll
-    for (int c = 0; c < TILE / 16; ++c) cp_async16(smem_u32(dst + 16 * c), src + 16 * c);
+    for (int c = 0; c < CHUNKS; ++c) cp_async16(smem_u32(dst + 16 * c), src + 16 * c);
     cp_async_arrive(bar);
   } else {
-    for (int c = 0; c < TILE / 4; ++c) {
+    for (int c = 0; c < 4 * CHUNKS; ++c) {
       uint32_t x = 0;
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const int64_t ii = i0 + c * 4 + b;
-        const uint32_t byte = (row < rows && ii < a.N) ? (uint32_t)__ldg(a.G + row * a.N + ii) : 0xFFu;
-        x |= byte << (8 * b);
+        const uint8_t* p = src + c * 4 + b;
+        x |= (p >= a.G && p < end ? (uint32_t)__ldg(p) : 0xFFu) << (8 * b);
       }
       *reinterpret_cast<uint32_t*>(dst + 4 * c) = x;
     }
     mbar_arrive(bar);
   }
+}
+
+// Offset (bytes) of a tile's first sample in row `lr` (0..31) of an unaligned G stage: tiles
+// start at packed rows and samples that are multiples of 16, so it is the same in every tile.
+static_assert(TILE % 64 == 0 && SNP_BLOCK % 64 == 0, "tiles start at packed rows that are multiples of 16");
+__device__ __forceinline__ uint32_t row_offset(const Args& a, int lr) {
+  return ((uint32_t)(reinterpret_cast<uintptr_t>(a.G) & 15) + (uint32_t)lr * (uint32_t)(a.N & 15)) & 15u;
 }
 
 // Converted Q tile (4096 B) into a shared-memory buffer by the producer warp: lane l copies
@@ -347,7 +369,7 @@ __device__ __forceinline__ void producer_load_q(const Args& a, int64_t tile, uin
   cp_async_arrive(bar);
 }
 
-template <bool F16>
+template <bool F16, bool AL>
 __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
   using F = Fmt<F16>;
   constexpr uint32_t ID_H = idesc(HALF, 0, 0, F::CODE);   // A = P (K-major), B = Q half (K-major)
@@ -370,7 +392,6 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
   const int r_eff = (int)min((int64_t)R, (a.M - jb + TILE - 1) / TILE);
   const int64_t s_first = split;
   const int n_my = (int)((a.n_stile - split + a.n_split - 1) / a.n_split);  // sample tiles of this CTA
-  const bool vec16 = (a.N & 15) == 0;
   const int nsteps = n_my * r_eff;
 
   // ---- prologue: TMEM (producer warp), barriers, P tiles (all threads)
@@ -473,8 +494,8 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
     if (n_my > 1) producer_load_q(a, s_first + a.n_split, sm + OFF_Q + P_TILE_BYTES, QFULL(1));
     int gst = 0, gr = 0, gsidx = 0, gstage = 0;  // next G load: step, SNP tile, sample tile, stage
     auto load_next_g = [&]() {
-      producer_load_g(a, (jb + (int64_t)gr * TILE) >> 2, (s_first + (int64_t)gsidx * a.n_split) * TILE,
-                      vec16, sm + OFF_G + gstage * G_TILE_BYTES, GFULL(gstage));
+      producer_load_g<AL>(a, (jb + (int64_t)gr * TILE) >> 2, (s_first + (int64_t)gsidx * a.n_split) * TILE,
+                          sm + OFF_G + gstage * G_TILE_BYTES, GFULL(gstage));
       ++gst;
       if (++gr == r_eff) { gr = 0; ++gsidx; }
       if (++gstage == NG) gstage = 0;
@@ -553,7 +574,11 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
     const int jl = wq * 32 + lane;              // SNP row within the tile
     const int colb = hw * HALF + sub * WG_COLS; // first sample column inside the step's tile
     const uint32_t trow = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(hw * 128 + sub * WG_COLS);
-    const uint32_t sh = 2u * (uint32_t)(jl & 3);
+    // bit shift of the SNP's field in a sample's byte; unaligned rows are read as words from
+    // the word at or below the thread's first sample, and one funnel shift takes off both
+    // the byte offset in the word and the field's position (at most 24 + 6 bits)
+    const uint32_t goff = AL ? 0u : row_offset(a, jl >> 2);
+    const uint32_t sh = 2u * (uint32_t)(jl & 3) + 8u * (goff & 3u);
     int r = 0, sidx = 0, gstage = 0;
     uint32_t hph = 0u, gph = 0u;
     for (int st = 0; st < nsteps; ++st) {
@@ -565,7 +590,7 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
       if (hw == 1 && sub == 0 && r == 0 && sidx > 0) write_t(s_first + (int64_t)(sidx - 1) * a.n_split);
 
       const int64_t jglob = jb + (int64_t)r * TILE + jl;
-      const uint8_t* gs = sm + OFF_G + gstage * G_TILE_BYTES + (jl >> 2) * G_ROW + colb;
+      const uint8_t* gs = sm + OFF_G + gstage * G_TILE_BYTES + (jl >> 2) * G_ROW + colb + (goff & ~3u);
       uint8_t* ta = sm + OFF_A + (st & 1) * AB_TILE_BYTES;
       uint8_t* tb = sm + OFF_B + (st & 1) * AB_TILE_BYTES;
       uint32_t hv[2][16], cv[2][16];
@@ -580,12 +605,18 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
           tmem_ld16(trow + HALF + 16 * (c + 1), cv[cur ^ 1]);
         }
         const int col0 = colb + 16 * c;
-        const uint4 gw = *reinterpret_cast<const uint4*>(gs + 16 * c);
-        const uint32_t words[4] = {gw.x, gw.y, gw.z, gw.w};
+        uint32_t words[5];
+        if constexpr (AL) {
+          const uint4 gw = *reinterpret_cast<const uint4*>(gs + 16 * c);
+          words[0] = gw.x; words[1] = gw.y; words[2] = gw.z; words[3] = gw.w; words[4] = 0;
+        } else {
+#pragma unroll
+          for (int q = 0; q < 5; ++q) words[q] = *reinterpret_cast<const uint32_t*>(gs + 16 * c + 4 * q);
+        }
         uint32_t ap[8], bp[8];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          uint32_t tq = (words[q] >> sh) & 0x03030303u;
+          uint32_t tq = (AL ? words[q] >> sh : __funnelshift_r(words[q], words[q + 1], sh)) & 0x03030303u;
           if (jglob >= a.M) tq = 0x03030303u;
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
@@ -756,20 +787,20 @@ int tc_plan(int64_t M, int64_t N, int K, int64_t& n_stile, int& n_split, int& n_
 
 size_t tc_q_bytes(int64_t n_stile) { return (size_t)n_stile * tc::P_TILE_BYTES; }
 
-template <bool F16>
+template <bool F16, bool AL>
 static int tc_launch(const tc::Args& a, int64_t n_stile, uint8_t* qb, const float* Q, cudaStream_t st) {
   static bool attr_set[64] = {false};
   int dev = 0;
   ADX_CUDA_TRY(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    ADX_CUDA_TRY(cudaFuncSetAttribute(tc::em_sweep_tc_kernel<F16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    ADX_CUDA_TRY(cudaFuncSetAttribute(tc::em_sweep_tc_kernel<F16, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       tc::SMEM_ALLOC));
     attr_set[dev] = true;
   }
   tc::q_to_tiles_kernel<F16><<<(unsigned)ceil_div(n_stile * tc::TILE * 2, 256), 256, 0, st>>>(Q, a.N, a.K,
                                                                                                 n_stile, qb);
   ADX_LAUNCH_CHECK();
-  tc::em_sweep_tc_kernel<F16><<<(unsigned)(a.n_split * a.n_mblk), tc::TPB, tc::SMEM_ALLOC, st>>>(a);
+  tc::em_sweep_tc_kernel<F16, AL><<<(unsigned)(a.n_split * a.n_mblk), tc::TPB, tc::SMEM_ALLOC, st>>>(a);
   ADX_LAUNCH_CHECK();
   return ADX_OK;
 }
@@ -789,7 +820,10 @@ int tc_sweep(const uint8_t* G, const float* P, const float* Q, int64_t M, int64_
              bool f16, cudaStream_t st) {
   uint8_t* qb = static_cast<uint8_t*>(Qb);
   const tc::Args a{G, P, qb, M, N, K, n_stile, n_split, n_mblk, ABp, Tp, err};
-  return f16 ? tc_launch<true>(a, n_stile, qb, Q, st) : tc_launch<false>(a, n_stile, qb, Q, st);
+  // aligned rows need one 16-byte shared load per 16 samples instead of five 4-byte ones
+  const bool al = (N & 15) == 0 && (reinterpret_cast<uintptr_t>(G) & 15) == 0;
+  if (f16) return al ? tc_launch<true, true>(a, n_stile, qb, Q, st) : tc_launch<true, false>(a, n_stile, qb, Q, st);
+  return al ? tc_launch<false, true>(a, n_stile, qb, Q, st) : tc_launch<false, false>(a, n_stile, qb, Q, st);
 }
 
 }  // namespace adx

@@ -45,3 +45,29 @@ def test_tensor_core_stats_do_not_depend_on_alignment(ops, prec, N, M):
         got = ops.em_stats(placed(packed, off), P32, Q32, M, prec)
         for g, r in zip(got, ref):
             assert torch.equal(g, r), off
+
+
+@pytest.mark.parametrize("N,M", [(1, 1), (3, 9), (15, 4), (16, 61), (17, 30), (511, 258), (528, 33), (4097, 70),
+                                 (9001, 1003)])
+def test_bed_and_statistics_do_not_depend_on_alignment(ops, N, M):
+    # BED decode (unit and segment edges, a flipped and an unflipped matrix), frequencies (warp
+    # and block per row) and per-sample counts (nibble, byte and 32-bit sums) at every kind
+    # of start address
+    for p in ([0.5, 0.25, 0.15, 0.1], [0.1, 0.2, 0.6, 0.1]):
+        G = np.random.default_rng(N * M).choice(4, size=(M, N), p=p).astype(np.uint8)
+        code = np.array([3, 2, 0, 1], dtype=np.uint8)[G]
+        pad = np.full((M, -N % 4), 1, dtype=np.uint8)      # what the padding holds must not matter
+        c = np.concatenate([code, pad], axis=1).reshape(M, -1, 4)
+        bed = c[..., 0] | c[..., 1] << 2 | c[..., 2] << 4 | c[..., 3] << 6
+        seen = G != 3
+        if seen.any() and (G * seen).sum() / (2.0 * seen.sum()) >= 0.5:
+            G = np.where(G == 0, 2, np.where(G == 2, 0, G)).astype(np.uint8)
+        packed = orc.pack(G)
+        cnt, tot = seen.sum(1), (G * seen).sum(1)
+        f = np.where(cnt > 0, tot.astype(np.float32) / np.float32(2) / np.maximum(cnt, 1).astype(np.float32), 0)
+        for off in (0, 1, 2, 7, 13):
+            assert torch.equal(ops.bed_to_packed(placed(bed, off), N, M).cpu(), torch.from_numpy(packed)), off
+            P = placed(packed, off)
+            np.testing.assert_allclose(ops.allele_frequency(P, M).cpu().numpy(), f, rtol=2.0 ** -22, atol=0)
+            assert np.array_equal(ops.sample_counts(P, M).cpu().numpy(), 2.0 * seen.sum(0))
+            assert np.array_equal(ops.sample_het_counts(P, M).cpu().numpy(), (G == 1).sum(0))

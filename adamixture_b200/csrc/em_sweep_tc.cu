@@ -54,7 +54,7 @@
 #include <queue>
 #include <vector>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 #ifndef ADX_TC_HALF_WGS
 #define ADX_TC_HALF_WGS 2
@@ -101,8 +101,6 @@ static_assert(SMEM_ALLOC < 256 * 1024, "descriptor start field");
 // TMEM columns
 constexpr uint32_t COL_T = 256, COL_AB = 272;
 
-constexpr uint32_t WAIT_LIMIT = 1u << 26;  // ~seconds of polling before giving up
-
 // ---------------------------------------------------------------- descriptors
 
 // Instruction descriptor, kind::f16: A/B format fmt (0 = FP16, 1 = BF16) for both, FP32 D,
@@ -110,12 +108,6 @@ constexpr uint32_t WAIT_LIMIT = 1u << 26;  // ~seconds of polling before giving 
 __host__ __device__ constexpr uint32_t idesc(int N, int a_mn, int b_mn, uint32_t fmt) {
   return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
          ((uint32_t)(N >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
-}
-
-// Shared-memory matrix descriptor, no swizzle, Blackwell version bit.
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
 // Byte offsets inside the tiles (element size 2).
@@ -130,10 +122,6 @@ __device__ __forceinline__ uint32_t off_ab(int j, int i) {
 
 // ---------------------------------------------------------------- PTX wrappers
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
 __device__ __forceinline__ void mma_f16kind(uint32_t tmem_d, uint64_t ad, uint64_t bd, uint32_t id,
                                             uint32_t accumulate) {
   asm volatile(
@@ -144,53 +132,6 @@ __device__ __forceinline__ void mma_f16kind(uint32_t tmem_d, uint64_t ad, uint64
       : "r"(tmem_d), "l"(ad), "l"(bd), "r"(id), "r"(accumulate));
 }
 
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait; returns false on timeout (raising the abort word) or when another warp has
-// aborted.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          uint32_t limit = WAIT_LIMIT) {
-  for (uint32_t it = 0; it < limit; ++it) {
-    if (mbar_try(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (it > 64) __nanosleep(32);
-  }
-  *abort_flag = 1;
-  return false;
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-// Arrive on `bar` once every cp.async this thread issued before has landed (the arrival
-// counts against the barrier's expected count).
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -200,8 +141,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
         "=r"(v[14]), "=r"(v[15])
       : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
 __device__ __forceinline__ float rcp_approx(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

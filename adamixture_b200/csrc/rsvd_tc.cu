@@ -1,0 +1,711 @@
+// Products of the centred genotype matrix with skinny float32 factors on the integer tensor
+// cores (tcgen05.mma kind::i8, 32-bit accumulators in tensor memory), for the shifted
+// randomized SVD (adamixture/model/svd_gpu.py:40-154):
+//
+//   rows:  Y[j] = sum_i x_ji B_i                    (x = g - 2 f_j, 0 where missing)
+//   cols:  Z[i] = sum_j x_ji Y_j
+//
+// A genotype code c is 0..3 (3: missing). With m = 1 where missing, g = c - 3m and the
+// centred entry is (c - 3m) - 2f (1 - m), so
+//   rows:  Y_j = (S1 - 3 S2) - 2 f_j (sum_i B_i - S2),   S1 = sum_i c B_i, S2 = sum_i m B_i
+//   cols:  Z_i = sum_j c y_j + sum_j m (2 f_j - 3) y_j - sum_j 2 f_j y_j
+// and every sum over the matrix is one of small integers (c, m) times a factor column. The
+// factor is taken to 31-bit fixed point relative to its column's largest magnitude and split
+// into four signed 8-bit digits (columns 4 x L of the B operand); products and sums are
+// exact in int32 (at most 3 x 128 x 4 Mi per digit and CTA), the CTAs' parts add exactly in
+// int64, and one rounding to float32 ends it. What is left is the quantization, at most 2^-31
+// of the column's largest magnitude per entry: 128 times finer than float32's own
+// rounding there. Against float64 the relative error is 2.5e-8 (the final rounding) where
+// float32 FMAs gave 5.6e-6 (N=100,000 x M=300,000). Columns with an infinity or a NaN, and SNPs with such
+// a frequency, are summed entry by entry in float32 instead (finalize kernels).
+//
+// CTA: 256 rows of the product (two 128-row MMA tiles) over a range of 256-entry blocks of
+// the contracted axis. Rows are SNPs and the contraction runs over samples, or the reverse:
+// either way a block is 64 packed rows x 256 samples of G. Two groups of 8 warps unpack, taking turns:
+// thread = row of the product; 64 entries at a time it forms the codes and the missing flags, 4 per 32-bit
+// register, and stores them to tensor memory, which feeds the MMAs' A operand: no unpacked
+// entry goes through shared memory. rows: a register is 4 samples of the SNP (one shift and
+// mask of the packed word); cols: the 4 SNPs of the sample's packed byte, spread to bytes.
+// One warp copies G (16-byte cp.async at any alignment, see row offsets) and the digit tiles
+// (bulk copies) into a 3-slot ring; another issues the MMAs. Tensor memory: accumulators
+// (2 tiles x {c, m} x 4 Lb columns), then a ring of 2 to 4 A stages of 64 columns. Lb, the factor
+// columns of a pass, is at most 24 so that two A stages fit; a wider factor takes
+// ceil(L / 24) passes of equal width.
+//
+// One pass each way at N=100,000 x M=300,000, L=20: 120.3 ms on float32 CUDA cores, 11.5 ms
+// here (the packed matrix read twice is 2.3 ms of HBM time).
+// What bounds it now is the hand-over of the A stages: with no MMAs issued the loop still takes
+// 60 % of the time, and each MMA adds the 50 cycles that it takes; the time does not depend on
+// L (16 to 24), nor on the loads, nor on the unpacking itself.
+#include "tcgen05.cuh"
+
+#include <math.h>
+
+namespace adx {
+namespace rt {
+
+using tc::cp_async16;
+using tc::cp_async_arrive;
+using tc::fence_after;
+using tc::fence_before;
+using tc::mbar_arrive;
+using tc::mma_commit;
+using tc::smem_u32;
+
+constexpr int TILE = 128;                 // rows of an MMA tile
+constexpr int OWN = 2 * TILE;             // rows of the product per CTA
+constexpr int BLK = 256;                  // contracted entries per block
+constexpr int KST = 64;                   // contracted entries per A stage
+constexpr int KSTEPS = BLK / KST;
+constexpr int NDIG = 4;                   // 8-bit digits per factor entry
+constexpr int LB_MAX = 24;                // factor columns per pass
+constexpr int L_MAX = 80;
+constexpr int NSLOT = 3;                  // G / digit slots
+constexpr int NSTAGE_MIN = 2, NSTAGE_MAX = 4;   // A stages
+constexpr int GROUPS = 2;                 // unpack groups, taking turns at the A stages
+constexpr int GROUP_WARPS = 8;            // a thread per row of the product
+constexpr int UNPACK_WARPS = GROUPS * GROUP_WARPS;
+static_assert(GROUPS <= KSTEPS, "every group works on every block");
+// A group waits for the MMAs of the stage's previous fill by that fill's parity, so it must
+// not come to a fill while the one before the previous is still to be read: its own last wait
+// (GROUPS stages ago, for MMAs nstage earlier still) proves that only if GROUPS <= nstage.
+static_assert(GROUPS <= NSTAGE_MIN, "a stage's fills cannot be confused by their parity");
+constexpr int LOAD_WARP = UNPACK_WARPS, MMA_WARP = UNPACK_WARPS + 1;
+constexpr int TPB = 32 * (UNPACK_WARPS + 2);
+constexpr int G_ROW = BLK + 16;           // bytes of a packed row in a slot, any alignment
+constexpr int G_BYTES = (OWN / 4) * G_ROW;
+constexpr int N_BARS = 2 * NSLOT + NSTAGE_MAX + 1;
+constexpr uint32_t POLLS = 1u << 22;      // of a bounded wait: a fraction of a second to a few seconds
+constexpr int64_t MAX_RED = int64_t(1) << 22;   // contracted entries per CTA: int32 sums are exact
+static_assert(OWN == BLK, "a block of G has the same shape in both products");
+static_assert(3ll * 128 * MAX_RED < (1ll << 31), "int32 digit sums");
+static_assert(2 * 2 * NDIG * LB_MAX + NSTAGE_MIN * 64 <= 512, "accumulators and the A stages in tensor memory");
+static_assert(G_ROW % 16 == 0 && G_BYTES % 16 == 0, "16-byte copies");
+
+struct Args {
+  const uint8_t* G;
+  int64_t M, N;
+  const uint8_t* dc;       // digit tiles of the codes' factor: [pass][block][256 x 4 Lb bytes]
+  const uint8_t* dm;       // of the flags' factor (rows: the same tiles)
+  int L, Lb, n_pass;
+  int64_t n_blk;           // contracted blocks
+  int64_t tiles;           // row tiles of 256
+  int n_split;             // ranges of the contracted axis
+  int nstage;
+  long long* sc;           // [rows][L] code sums (rows: S1 - 3 S2)
+  long long* sm;           // [rows][L] flag sums
+  int* err;
+};
+
+__host__ __device__ inline int digit_bytes(int Lb) { return BLK * NDIG * Lb; }
+
+// Instruction descriptor, kind::i8: D int32, A and B signed 8-bit, both K-major, M = 128.
+__device__ __forceinline__ uint32_t idesc_i8(int n) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
+}
+
+// D (tensor memory) += A (tensor memory) . B (shared memory), M=128, K=32.
+__device__ __forceinline__ void mma_i8(uint32_t d, uint32_t a, uint64_t bd, uint32_t id, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}\n"
+      :
+      : "r"(d), "r"(a), "l"(bd), "r"(id), "r"(accumulate));
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      :
+      : "r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t (&v)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"(addr));
+}
+
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               :
+               : "r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void arrive_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar),
+               "r"(bytes)
+               : "memory");
+}
+
+// Bounded wait of a whole warp. It never blocks once the CTA has given up (a timeout raises
+// the abort word): every warp then runs its loop to the end without waiting, so that each
+// named barrier still gets all its arrivals, and the result is discarded.
+__device__ __forceinline__ void warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  for (uint32_t it = 0; it < POLLS; ++it) {
+    if (tc::mbar_try(bar, parity)) return;
+    if ((it & 15u) == 15u && *abort_flag) return;
+  }
+  *abort_flag = 1;
+}
+
+// A stage's hand-over from the unpack group to the MMA warp: a named barrier (a hardware
+// barrier wakes the waiter in tens of cycles; an mbarrier here cost several hundred per stage).
+constexpr int HANDOVER = 32 * (GROUP_WARPS + 1);
+__device__ __forceinline__ void stage_arrive(int st) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(1 + st), "n"(HANDOVER) : "memory");
+}
+__device__ __forceinline__ void stage_sync(int st) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + st), "n"(HANDOVER) : "memory");
+}
+
+// 64 packed rows from row0 x 256 samples from i0 into a slot, by the load warp. AL: every
+// packed row starts 16-byte aligned, 16 chunks a row; otherwise 17 chunks from the 16-byte
+// boundary at or below the row's first byte (readers add row_offset). Chunks that would
+// leave the matrix take byte loads (0 past the ends); rows past the matrix are not loaded.
+// What is read for samples past N or SNPs past M does not matter: their digits are zero, or
+// their product rows are not stored.
+template <bool AL>
+__device__ __forceinline__ void load_g(const Args& a, int64_t row0, int64_t i0, uint8_t* gs) {
+  const int lane = threadIdx.x & 31;
+  const int64_t rows = (a.M + 3) >> 2;
+  const uint8_t* end = a.G + rows * a.N;
+  auto chunk = [&](int r, int c) {
+    const int64_t row = row0 + r;
+    if (row >= rows) return;
+    const uint8_t* src = a.G + row * a.N + i0;
+    if constexpr (!AL) src -= reinterpret_cast<uintptr_t>(src) & 15;
+    src += 16 * c;
+    uint8_t* dst = gs + r * G_ROW + 16 * c;
+    if (src >= a.G && src + 16 <= end) {
+      cp_async16(smem_u32(dst), src);
+    } else {
+      for (int b = 0; b < 16; ++b) dst[b] = src + b >= a.G && src + b < end ? __ldg(src + b) : (uint8_t)0;
+    }
+  };
+  const uint8_t* first = a.G + row0 * a.N + i0;
+  // a block inside the matrix (and 16 bytes either way): one pointer walks the rows. The
+  // general form's checks and 64-bit products, about 25 instructions a chunk in one warp, were
+  // what the whole kernel waited for (3.4 ms a pass against 2.4 at N = M = 100,000)
+  if (row0 + OWN / 4 <= rows && first - 16 >= a.G && first + (OWN / 4 - 1) * a.N + BLK + 16 <= end) {
+    const uint8_t* src = first + (lane >> 4) * a.N + 16 * (lane & 15);
+    uint32_t dst = smem_u32(gs) + (uint32_t)(lane >> 4) * G_ROW + 16u * (uint32_t)(lane & 15);
+    const int64_t step = 2 * a.N;
+#pragma unroll 8
+    for (int r = 0; r < OWN / 4; r += 2, src += step, dst += 2 * G_ROW)
+      cp_async16(dst, AL ? src : src - (reinterpret_cast<uintptr_t>(src) & 15));
+    if constexpr (!AL) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint8_t* s16 = first + (lane + 32 * h) * a.N + BLK;
+        cp_async16(smem_u32(gs) + (uint32_t)(lane + 32 * h) * G_ROW + BLK, s16 - (reinterpret_cast<uintptr_t>(s16) & 15));
+      }
+    }
+    return;
+  }
+  for (int e = lane; e < (OWN / 4) * (BLK / 16); e += 32) chunk(e / (BLK / 16), e % (BLK / 16));
+  if constexpr (!AL) {
+    chunk(lane, BLK / 16);
+    chunk(lane + 32, BLK / 16);
+  }
+}
+
+// Offset (bytes) of a block's first sample in its packed row lr: blocks start at packed rows
+// and samples that are multiples of 16, so it depends on lr mod 16 alone.
+__device__ __forceinline__ uint32_t row_offset(const Args& a, int lr) {
+  return ((uint32_t)(reinterpret_cast<uintptr_t>(a.G) & 15) + (uint32_t)lr * (uint32_t)(a.N & 15)) & 15u;
+}
+
+template <bool ROWS, bool AL>
+__global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n4 = NDIG * a.Lb;
+  const uint32_t dbytes = (uint32_t)digit_bytes(a.Lb);
+  const uint32_t slot_bytes = G_BYTES + (ROWS ? 1u : 2u) * dbytes;
+  uint8_t* ctl = sm + NSLOT * slot_bytes;
+  const uint32_t bars = smem_u32(ctl);
+  auto FULL = [&](int s) { return bars + 8u * (uint32_t)s; };
+  auto EMPTY = [&](int s) { return bars + 8u * (uint32_t)(NSLOT + s); };
+  auto AEMPTY = [&](int s) { return bars + 8u * (uint32_t)(2 * NSLOT + s); };
+  const uint32_t DONE = bars + 8u * (uint32_t)(N_BARS - 1);
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(ctl + 8 * N_BARS);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(ctl + 8 * N_BARS + 4);
+
+  int64_t b = blockIdx.x;
+  const int64_t tile = b % a.tiles; b /= a.tiles;
+  const int split = (int)(b % a.n_split);
+  const int pass = (int)(b / a.n_split);
+  const int64_t per = (a.n_blk + a.n_split - 1) / a.n_split;
+  const int64_t q0 = (int64_t)split * per;
+  const int nq = (int)(min(a.n_blk, q0 + per) - q0);   // at least 1: the host's n_split is exact
+
+  if (warp == MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_holder)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < NSLOT; ++s) {
+      // 32 asynchronous and 32 plain arrivals of the load warp, and the bulk copies' expect
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 65;" ::"r"(FULL(s)));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(EMPTY(s)));
+    }
+    for (int s = 0; s < NSTAGE_MAX; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(AEMPTY(s)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(DONE));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = *tmem_holder;
+  const uint32_t col_a = tmem + 4u * (uint32_t)n4;      // A stages: per stage and tile 16 code, 16 flag columns
+
+  if (warp == LOAD_WARP) {
+    int slot = 0;
+    uint32_t fill = 0;   // how often the ring has wrapped
+    for (int q = 0; q < nq; ++q) {
+      if (fill > 0) warp_wait(EMPTY(slot), (fill - 1) & 1u, abort_flag);
+      uint8_t* gs = sm + slot * slot_bytes;
+      const int64_t blk = q0 + q;
+      if (lane == 0) {
+        arrive_expect(FULL(slot), (ROWS ? 1u : 2u) * dbytes);
+        const int64_t at = ((int64_t)pass * a.n_blk + blk) * dbytes;
+        bulk_copy(smem_u32(gs + G_BYTES), a.dc + at, dbytes, FULL(slot));
+        if constexpr (!ROWS) bulk_copy(smem_u32(gs + G_BYTES + dbytes), a.dm + at, dbytes, FULL(slot));
+      }
+      load_g<AL>(a, (ROWS ? tile * OWN : blk * BLK) >> 2, ROWS ? blk * BLK : tile * OWN, gs);
+      cp_async_arrive(FULL(slot));
+      mbar_arrive(FULL(slot));
+      if (++slot == NSLOT) { slot = 0; ++fill; }
+    }
+  } else if (warp == MMA_WARP) {
+    const uint32_t id = idesc_i8(n4);
+    int slot = 0, st = 0;
+    uint32_t fill = 0;
+    for (int q = 0; q < nq; ++q) {
+      warp_wait(FULL(slot), fill & 1u, abort_flag);
+      const uint32_t sb = smem_u32(sm + slot * slot_bytes + G_BYTES);
+      const uint64_t dc = tc::sdesc(sb, 128, 256), dm = ROWS ? dc : tc::sdesc(sb + dbytes, 128, 256);
+      const uint64_t step = (uint64_t)(32 * n4) >> 4;   // one 32-entry step of a digit tile
+      for (int ks = 0; ks < KSTEPS; ++ks) {
+        stage_sync(st);
+        fence_after();
+        if (lane == 0) {
+          const uint32_t as = col_a + 64u * (uint32_t)st;
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) {
+            const uint64_t off = step * (uint64_t)(2 * ks + kk);
+            const uint32_t acc = (q > 0 || ks > 0 || kk > 0) ? 1u : 0u;
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+              mma_i8(tmem + (uint32_t)(2 * t * n4), as + 32u * t + 8u * kk, dc + off, id, acc);
+              mma_i8(tmem + (uint32_t)((2 * t + 1) * n4), as + 32u * t + 16u + 8u * kk, dm + off, id, acc);
+            }
+          }
+          mma_commit(AEMPTY(st));
+          if (ks == KSTEPS - 1) mma_commit(EMPTY(slot));
+        }
+        __syncwarp();
+        if (++st == a.nstage) st = 0;
+      }
+      if (++slot == NSLOT) { slot = 0; ++fill; }
+    }
+    if (lane == 0) mma_commit(DONE);
+    __syncwarp();
+  } else {
+    const int wq = warp & 3, t = (warp >> 2) & 1, grp = warp / GROUP_WARPS;
+    const int own = t * TILE + wq * 32 + lane;        // row of the product within the CTA
+    const uint32_t lanes = (uint32_t)(wq * 32) << 16;
+    uint32_t goff[ROWS ? 1 : 16];                     // byte offsets into a slot
+    uint32_t sh = 0;
+    if constexpr (ROWS) {
+      const uint32_t o = AL ? 0u : row_offset(a, own >> 2);
+      goff[0] = (uint32_t)(own >> 2) * G_ROW + (o & ~3u);
+      sh = 2u * (uint32_t)(own & 3) + 8u * (o & 3u);
+    } else {
+#pragma unroll
+      for (int p = 0; p < 16; ++p) goff[p] = (uint32_t)p * G_ROW + (AL ? 0u : row_offset(a, p)) + (uint32_t)own;
+    }
+    int slot = 0, st = 0, turn = 0;
+    uint32_t fill = 0, sfill = 0;
+    for (int q = 0; q < nq; ++q) {
+      warp_wait(FULL(slot), fill & 1u, abort_flag);
+      const uint8_t* gs = sm + slot * slot_bytes;
+      for (int ks = 0; ks < KSTEPS; ++ks) {
+        const bool mine = turn == grp;
+        if (++turn == GROUPS) turn = 0;
+        const int my_st = st;
+        const uint32_t my_fill = sfill;
+        if (++st == a.nstage) { st = 0; ++sfill; }
+        if (!mine) continue;
+        uint32_t x[16], m[16];
+        if constexpr (ROWS) {
+          const uint8_t* src = gs + goff[0] + KST * ks;
+          if constexpr (AL) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const uint4 v = *reinterpret_cast<const uint4*>(src + 16 * c);
+              x[4 * c] = v.x >> sh; x[4 * c + 1] = v.y >> sh; x[4 * c + 2] = v.z >> sh; x[4 * c + 3] = v.w >> sh;
+            }
+          } else {
+            uint32_t w = *reinterpret_cast<const uint32_t*>(src);
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+              const uint32_t nx = *reinterpret_cast<const uint32_t*>(src + 4 * c + 4);
+              x[c] = __funnelshift_r(w, nx, sh);
+              w = nx;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int p = 0; p < 16; ++p) {
+            // the byte's fields to the low bits of four bytes
+            const uint32_t v = (uint32_t)gs[goff[p] + (uint32_t)(16 * ks * G_ROW)] * 0x1001u;
+            x[p] = v | (v << 6);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          x[c] &= 0x03030303u;
+          m[c] = x[c] & (x[c] >> 1) & 0x01010101u;
+        }
+        if (my_fill > 0) warp_wait(AEMPTY(my_st), (my_fill - 1) & 1u, abort_flag);
+        fence_after();
+        const uint32_t as = col_a + lanes + 64u * (uint32_t)my_st + 32u * (uint32_t)t;
+        tmem_st16(as, x);
+        tmem_st16(as + 16, m);
+        tmem_wait_st();
+        fence_before();
+        stage_arrive(my_st);
+      }
+      if (++slot == NSLOT) { slot = 0; ++fill; }
+    }
+  }
+  warp_wait(DONE, 0u, abort_flag);
+  if (__syncthreads_or(*abort_flag)) {
+    // a bounded wait ran out: before the block ends, the copies and MMAs in flight land (these
+    // waits are bounded too)
+    if (tid == 0) atomicExch(a.err, ADX_ERR_TIMEOUT);
+    if (warp == LOAD_WARP) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      volatile int never = 0;
+      for (int s = 0; s < NSLOT; ++s) {
+        const int fills = (nq - s + NSLOT - 1) / NSLOT;
+        if (fills > 0) warp_wait(FULL(s), (uint32_t)(fills - 1) & 1u, &never);
+      }
+      warp_wait(DONE, 0u, &never);
+    }
+  } else {
+    fence_after();
+    if (warp < GROUP_WARPS) {
+      const int wq = warp & 3, t = warp >> 2;
+      const int64_t row = tile * OWN + t * TILE + wq * 32 + lane;
+      const int64_t n_rows = ROWS ? a.M : a.N;
+      const uint32_t at = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(2 * t * n4);
+      for (int l = 0; l < a.Lb; l += 4) {
+        uint32_t v[2][NDIG][4];
+#pragma unroll
+        for (int o = 0; o < 2; ++o)
+#pragma unroll
+          for (int d = 0; d < NDIG; ++d) tmem_ld4(at + (uint32_t)(o * n4 + d * a.Lb + l), v[o][d]);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int lg = pass * a.Lb + l + e;
+          long long s[2];
+#pragma unroll
+          for (int o = 0; o < 2; ++o) {
+            s[o] = (int)v[o][NDIG - 1][e];
+#pragma unroll
+            for (int d = NDIG - 2; d >= 0; --d) s[o] = s[o] * 256 + (int)v[o][d][e];
+          }
+          if (ROWS) s[0] -= 3 * s[1];
+          if (row < n_rows && lg < a.L) {
+            const int64_t w = row * a.L + lg;
+            if (a.n_split == 1) {
+              a.sc[w] = s[0];
+              a.sm[w] = s[1];
+            } else {   // integers: the order does not matter
+              atomicAdd(reinterpret_cast<unsigned long long*>(a.sc + w), (unsigned long long)s[0]);
+              atomicAdd(reinterpret_cast<unsigned long long*>(a.sm + w), (unsigned long long)s[1]);
+            }
+          }
+        }
+      }
+    }
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  if (warp == MMA_WARP) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+  }
+}
+
+// ---------------------------------------------------------------- factors to digits
+
+// The factors of a product, from F [n][L]: codes take F; flags take F (rows) or (2f - 3) F
+// (cols, f per entry); the constant sum takes F (rows) or 2 f F (cols).
+template <bool ROWS>
+__device__ __forceinline__ double factor(int which, float y, float f) {
+  if (ROWS || which == 0) return (double)y;
+  const double u = 2.0 * (double)f * (double)y;
+  return which == 1 ? u - 3.0 * (double)y : u;
+}
+constexpr int N_FACT = 3;       // codes, flags, constant sum
+constexpr int SUM_BITS = 36;    // fixed point of the cols product's constant sum
+
+// Head of the workspace: largest magnitudes (float bits), constant sums, status.
+struct Head {
+  uint32_t top[N_FACT][L_MAX];
+  unsigned long long csum[L_MAX];
+  int err;
+};
+
+// 2^bits over a power of two above the column's largest magnitude.
+__device__ __forceinline__ double quantum_inv(uint32_t top, int bits) {
+  return top ? ldexp(1.0, bits - 1 - ilogbf(__uint_as_float(top))) : 0.0;
+}
+__device__ __forceinline__ bool finite_bits(uint32_t top) { return top < 0x7F800000u; }
+
+template <bool ROWS>
+__global__ void __launch_bounds__(256) top_kernel(const float* __restrict__ F, const float* __restrict__ f, int64_t n,
+                                                  int L, Head* h) {
+  __shared__ uint32_t top[N_FACT][L_MAX];
+  for (int e = threadIdx.x; e < N_FACT * L_MAX; e += 256) top[e / L_MAX][e % L_MAX] = 0;
+  __syncthreads();
+  const int per = 256 / L, l = threadIdx.x % L, g = threadIdx.x / L;
+  if (g < per) {
+    uint32_t t[N_FACT] = {0, 0, 0};
+    for (int64_t i = (int64_t)blockIdx.x * per + g; i < n; i += (int64_t)gridDim.x * per) {
+      const float y = F[i * L + l], fi = ROWS ? 0.0f : f[i];
+      // the magnitudes' bits order as the magnitudes do, a NaN's above all
+#pragma unroll
+      for (int w = 0; w < (ROWS ? 1 : N_FACT); ++w)
+        t[w] = max(t[w], __float_as_uint((float)factor<ROWS>(w, y, fi)) & 0x7FFFFFFFu);
+    }
+#pragma unroll
+    for (int w = 0; w < (ROWS ? 1 : N_FACT); ++w) atomicMax(&top[w][l], t[w]);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < (ROWS ? 1 : N_FACT) * L; e += 256)
+    atomicMax(&h->top[e / L][e % L], top[e / L][e % L]);
+}
+
+// Thread per (16 contracted entries, factor column): 16 bytes of each digit, in the order of
+// the shared-memory tile (32-entry steps of 4 Lb x 32 bytes: core matrices of 8 columns x 16
+// entries). Entries past n and columns past L are zero.
+template <bool ROWS>
+__global__ void __launch_bounds__(256) digit_kernel(const float* __restrict__ F, const float* __restrict__ f,
+                                                    int64_t n, int L, int Lb, int n_pass, int64_t n_blk, Head* h,
+                                                    uint8_t* __restrict__ dc, uint8_t* __restrict__ dm) {
+  __shared__ unsigned long long csum[L_MAX];
+  for (int e = threadIdx.x; e < L_MAX; e += 256) csum[e] = 0;
+  __syncthreads();
+  const int cols = n_pass * Lb;
+  const int64_t work = n_blk * (BLK / 16) * cols;
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < work; e += (int64_t)gridDim.x * 256) {
+    const int64_t kg = e / cols;
+    const int lg = (int)(e - kg * cols), pass = lg / Lb, lc = lg - pass * Lb;
+    const bool on = lg < L && finite_bits(h->top[0][lg]) && (ROWS || (finite_bits(h->top[1][lg]) && finite_bits(h->top[2][lg])));
+    double inv[N_FACT] = {0.0, 0.0, 0.0};
+    if (on) {
+      inv[0] = quantum_inv(h->top[0][lg], 30);
+      if (!ROWS) {
+        inv[1] = quantum_inv(h->top[1][lg], 30);
+        inv[2] = quantum_inv(h->top[2][lg], SUM_BITS);
+      }
+    }
+    long long c = 0;
+    uint32_t dig[2][NDIG][4] = {};
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const int64_t i = kg * 16 + k;
+      const bool in = on && i < n;
+      const float y = in ? F[i * L + lg] : 0.0f, fi = !ROWS && in ? f[i] : 0.0f;
+#pragma unroll
+      for (int w = 0; w < (ROWS ? 1 : 2); ++w) {
+        int q = __double2int_rn(factor<ROWS>(w, y, fi) * inv[w]);
+        if (ROWS) c += q;
+#pragma unroll
+        for (int d = 0; d < NDIG; ++d) {
+          const int lo = (int)(int8_t)(q & 0xFF);   // signed digit; the rest divides exactly
+          dig[w][d][k >> 2] |= (uint32_t)(lo & 0xFF) << (8 * (k & 3));
+          q = (q - lo) >> 8;
+        }
+      }
+      if (!ROWS) c += __double2ll_rn(factor<ROWS>(2, y, fi) * inv[2]);
+    }
+    if (on) atomicAdd(&csum[lg], (unsigned long long)c);
+    const int64_t base = ((int64_t)pass * n_blk * (BLK / 32) + (kg >> 1)) * (32 * NDIG * Lb);
+#pragma unroll
+    for (int d = 0; d < NDIG; ++d) {
+      const int col = d * Lb + lc;
+      const int64_t at = base + (col >> 3) * 256 + (kg & 1) * 128 + (col & 7) * 16;
+      *reinterpret_cast<uint4*>(dc + at) = make_uint4(dig[0][d][0], dig[0][d][1], dig[0][d][2], dig[0][d][3]);
+      if (!ROWS) *reinterpret_cast<uint4*>(dm + at) = make_uint4(dig[1][d][0], dig[1][d][1], dig[1][d][2], dig[1][d][3]);
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < L; e += 256)
+    if (csum[e]) atomicAdd(&h->csum[e], csum[e]);
+}
+
+// One thread per output element: the integer sums to float32. Elements whose factor column
+// or frequency is not finite are summed directly, as float32 arithmetic would have them.
+template <bool ROWS>
+__global__ void __launch_bounds__(256) finalize_kernel(const uint8_t* __restrict__ G, int64_t M, int64_t N,
+                                                       const float* __restrict__ F, const float* __restrict__ f, int L,
+                                                       const long long* __restrict__ sc,
+                                                       const long long* __restrict__ sm, const Head* __restrict__ h,
+                                                       int accumulate, float* __restrict__ out) {
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const int64_t n_rows = ROWS ? M : N;
+  if (e >= n_rows * L) return;
+  const int64_t row = e / L;
+  const int l = (int)(e - row * L);
+  const uint32_t t0 = h->top[0][l], t1 = h->top[1][l], t2 = h->top[2][l];
+  const float fr = ROWS ? f[row] : 0.0f;
+  float v;
+  if (h->err) {
+    v = __uint_as_float(0x7FFFFFFFu);   // a bounded wait ran out: not a result
+  } else if (!finite_bits(t0) || !finite_bits(t1) || !finite_bits(t2) || (ROWS && !isfinite(fr))) {
+    v = 0.0f;
+    for (int64_t r = 0; r < (ROWS ? N : M); ++r) {
+      const int64_t j = ROWS ? row : r, i = ROWS ? r : row;
+      const unsigned g = genotype(G[(j >> 2) * N + i], (int)(j & 3));
+      const float x = g == 3u ? 0.0f : (float)g - 2.0f * f[j];
+      v = fmaf(x, F[r * L + l], v);
+    }
+  } else if (ROWS) {
+    const double q = t0 ? 1.0 / quantum_inv(t0, 30) : 0.0;
+    v = (float)(q * ((double)sc[e] - 2.0 * (double)fr * (double)((long long)h->csum[l] - sm[e])));
+  } else {
+    const double q0 = t0 ? 1.0 / quantum_inv(t0, 30) : 0.0, q1 = t1 ? 1.0 / quantum_inv(t1, 30) : 0.0;
+    const double q2 = t2 ? 1.0 / quantum_inv(t2, SUM_BITS) : 0.0;
+    v = (float)(q0 * (double)sc[e] + q1 * (double)sm[e] - q2 * (double)(long long)h->csum[l]);
+  }
+  out[e] = accumulate ? out[e] + v : v;
+}
+
+// ---------------------------------------------------------------- plan
+
+constexpr size_t ALIGN = 256;   // of the workspace's parts (bulk copies read from it); any caller's pointer will do
+
+struct Plan {
+  int Lb, n_pass, n_split, nstage;
+  int64_t n_blk, tiles;
+  size_t head, digits, sums, bytes;   // bytes of each part and in all
+};
+
+// Splits of the contracted axis: the count whose CTAs (one per SM) finish first, counting
+// blocks and about 3 blocks of prologue and epilogue per CTA; the smallest of equals.
+static Plan plan(int64_t n_rows, int64_t n_red, int L, bool rows) {
+  Plan p{};
+  p.n_pass = (L + LB_MAX - 1) / LB_MAX;
+  p.Lb = ((L + p.n_pass - 1) / p.n_pass + 3) / 4 * 4;
+  p.n_blk = ceil_div(n_red, BLK);
+  p.tiles = ceil_div(n_rows, OWN);
+  const int fit = (512 - 4 * NDIG * p.Lb) / 64;
+  p.nstage = fit < NSTAGE_MAX ? fit : NSTAGE_MAX;
+  const int64_t sms = 148;
+  const int64_t lo = ceil_div(p.n_blk * BLK, MAX_RED);
+  const int64_t hi = p.n_blk < lo + 255 ? p.n_blk : lo + 255;
+  int64_t best = -1;
+  for (int64_t s = lo; s <= hi; ++s) {
+    const int64_t per = ceil_div(p.n_blk, s);
+    if (ceil_div(p.n_blk, per) != s) continue;   // the same ranges as a smaller count
+    const int64_t t = ceil_div(p.tiles * p.n_pass * s, sms) * (per + 3);
+    if (best < 0 || t < best) { best = t; p.n_split = (int)s; }
+  }
+  auto pad = [](size_t b) { return (b + ALIGN - 1) & ~(ALIGN - 1); };
+  p.head = pad(sizeof(Head));
+  p.digits = pad((size_t)p.n_pass * p.n_blk * digit_bytes(p.Lb));
+  p.sums = pad((size_t)n_rows * L * sizeof(long long));
+  p.bytes = p.head + (rows ? 1 : 2) * p.digits + 2 * p.sums + ALIGN;
+  return p;
+}
+
+template <bool ROWS, bool AL>
+static int launch(const Args& a, cudaStream_t st) {
+  // one CTA per SM: it takes the SM's tensor memory
+  const size_t need = (size_t)NSLOT * (G_BYTES + (ROWS ? 1 : 2) * digit_bytes(a.Lb)) + 8 * N_BARS + 16 + 128;
+  const size_t smem = need > 120 * 1024 ? need : 120 * 1024;
+  ADX_CUDA_TRY(cudaFuncSetAttribute(product_kernel<ROWS, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  product_kernel<ROWS, AL><<<(unsigned)(a.tiles * a.n_split * a.n_pass), TPB, smem, st>>>(a);
+  ADX_LAUNCH_CHECK();
+  return ADX_OK;
+}
+static_assert(NSLOT * (G_BYTES + 2 * BLK * NDIG * LB_MAX) + 8 * N_BARS + 16 + 128 <= 227 * 1024, "shared memory");
+
+template <bool ROWS>
+static int product(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* F, int L, int accumulate,
+                   float* out, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  const int64_t n_rows = ROWS ? M : N, n_red = ROWS ? N : M;
+  const Plan p = plan(n_rows, n_red, L, ROWS);
+  if (!workspace || workspace_bytes < p.bytes) return ADX_ERR_WORKSPACE;
+  uint8_t* w = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(workspace) + ALIGN - 1) & ~uintptr_t(ALIGN - 1));
+  Head* h = reinterpret_cast<Head*>(w);
+  uint8_t* dc = w + p.head;
+  uint8_t* dm = ROWS ? dc : dc + p.digits;
+  long long* sc = reinterpret_cast<long long*>(dm + p.digits);
+  long long* sm = reinterpret_cast<long long*>(reinterpret_cast<uint8_t*>(sc) + p.sums);
+  ADX_CUDA_TRY(cudaMemsetAsync(h, 0, sizeof(Head), st));
+  if (p.n_split > 1) ADX_CUDA_TRY(cudaMemsetAsync(sc, 0, 2 * p.sums, st));
+  const int64_t cap = (int64_t)sm_count() * 8;
+  const int64_t tb = ceil_div(n_red, 8 * (256 / L)), db = ceil_div(p.n_blk * (BLK / 16) * p.n_pass * p.Lb, 256);
+  top_kernel<ROWS><<<(unsigned)(tb < cap ? tb : cap), 256, 0, st>>>(F, f, n_red, L, h);
+  ADX_LAUNCH_CHECK();
+  digit_kernel<ROWS><<<(unsigned)(db < cap ? db : cap), 256, 0, st>>>(F, f, n_red, L, p.Lb, p.n_pass, p.n_blk, h, dc, dm);
+  ADX_LAUNCH_CHECK();
+  const Args a{G, M, N, dc, dm, L, p.Lb, p.n_pass, p.n_blk, p.tiles, p.n_split, p.nstage, sc, sm, &h->err};
+  const bool al = (N & 15) == 0 && (reinterpret_cast<uintptr_t>(G) & 15) == 0;
+  const int rc = al ? launch<ROWS, true>(a, st) : launch<ROWS, false>(a, st);
+  if (rc) return rc;
+  finalize_kernel<ROWS><<<(unsigned)ceil_div(n_rows * L, 256), 256, 0, st>>>(G, M, N, F, f, L, sc, sm, h, accumulate, out);
+  ADX_LAUNCH_CHECK();
+  return ADX_OK;
+}
+
+}  // namespace rt
+}  // namespace adx
+
+using namespace adx;
+
+extern "C" int adx_rsvd_workspace_bytes(int64_t M, int64_t N, int L, size_t* bytes) {
+  if (!bytes || M <= 0 || N <= 0 || L < 1 || L > rt::L_MAX) {
+    adx_set_message("adx_rsvd_workspace_bytes: bad argument");
+    return ADX_ERR_ARG;
+  }
+  const size_t r = rt::plan(M, N, L, true).bytes, c = rt::plan(N, M, L, false).bytes;
+  *bytes = r > c ? r : c;
+  return ADX_OK;
+}
+
+extern "C" int adx_rsvd_rows_ws(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* B, int L,
+                                float* Y, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!G || !f || !B || !Y || M <= 0 || N <= 0 || L < 1 || L > rt::L_MAX) {
+    adx_set_message("adx_rsvd_rows_ws: bad argument");
+    return ADX_ERR_ARG;
+  }
+  const int rc = rt::product<true>(G, M, N, f, B, L, 0, Y, workspace, workspace_bytes, as_stream(stream));
+  if (rc == ADX_ERR_WORKSPACE) adx_set_message("adx_rsvd_rows_ws: workspace too small");
+  return rc;
+}
+
+extern "C" int adx_rsvd_cols(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* Y, int L,
+                             int accumulate, float* Z, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!G || !f || !Y || !Z || M <= 0 || N <= 0 || L < 1 || L > rt::L_MAX) {
+    adx_set_message("adx_rsvd_cols: bad argument");
+    return ADX_ERR_ARG;
+  }
+  const int rc = rt::product<false>(G, M, N, f, Y, L, accumulate, Z, workspace, workspace_bytes, as_stream(stream));
+  if (rc == ADX_ERR_WORKSPACE) adx_set_message("adx_rsvd_cols: workspace too small");
+  return rc;
+}

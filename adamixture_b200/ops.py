@@ -477,6 +477,12 @@ def register_reference_ops() -> None:
 
 # ---------------------------------------------------------------- initialisation
 
+def _rsvd_workspace(device: torch.device, M: int, N: int, L: int) -> torch.Tensor:
+    """Scratch of one product, the call's own (the caching allocator keeps it to the current
+    stream), so products on several streams or threads do not share it."""
+    return torch.empty(query_size("adx_rsvd_workspace_bytes", M, N, L), dtype=torch.uint8, device=device)
+
+
 def rsvd_rows(G: torch.Tensor, f: torch.Tensor, B: torch.Tensor, M: int,
               out: torch.Tensor | None = None) -> torch.Tensor:
     """``Xc @ B`` for the centred genotypes (float32 ``[M, L]``), B float32 ``[N, L]``."""
@@ -486,8 +492,9 @@ def rsvd_rows(G: torch.Tensor, f: torch.Tensor, B: torch.Tensor, M: int,
     N, L = B.shape
     Y = torch.empty((M, L), dtype=torch.float32, device=G.device) if out is None else out
     _check(Y, "out", torch.float32, G.device)
-    call("adx_rsvd_rows", G.data_ptr(), M, N, f.data_ptr(), B.data_ptr(), L, Y.data_ptr(),
-         _stream(G.device))
+    ws = _rsvd_workspace(G.device, M, N, L)
+    call("adx_rsvd_rows_ws", G.data_ptr(), M, N, f.data_ptr(), B.data_ptr(), L, Y.data_ptr(),
+         ws.data_ptr(), ws.numel(), _stream(G.device))
     return Y
 
 
@@ -501,8 +508,7 @@ def rsvd_cols(G: torch.Tensor, f: torch.Tensor, Y: torch.Tensor, M: int,
     L = Y.shape[1]
     Z = torch.empty((N, L), dtype=torch.float32, device=G.device) if out is None else out
     _check(Z, "out", torch.float32, G.device)
-    nb = query_size("adx_rsvd_workspace_bytes", M, N, L)
-    ws = Workspace.get(G.device, nb, "rsvd")
+    ws = _rsvd_workspace(G.device, M, N, L)
     call("adx_rsvd_cols", G.data_ptr(), M, N, f.data_ptr(), Y.data_ptr(), L, int(bool(accumulate)),
          Z.data_ptr(), ws.data_ptr(), ws.numel(), _stream(G.device))
     return Z

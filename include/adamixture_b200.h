@@ -259,8 +259,12 @@ int adx_loglik_noalloc(const uint8_t* G, int64_t M, int64_t N, int K, int precis
 int adx_rsvd_rows(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* B, int L,
                   float* Y, void* stream);
 int adx_rsvd_workspace_bytes(int64_t M, int64_t N, int L, size_t* bytes);
-/* Z[N][L] = Xc' Y (accumulate != 0: Z += Xc' Y), Y float32 [M][L]; partial sums in the
- * workspace are added in a fixed order. */
+/* The same with a workspace (adx_rsvd_workspace_bytes, any alignment): on the integer tensor
+ * cores, from the factor in 31-bit fixed point. */
+int adx_rsvd_rows_ws(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* B, int L,
+                     float* Y, void* workspace, size_t workspace_bytes, void* stream);
+/* Z[N][L] = Xc' Y (accumulate != 0: Z += Xc' Y), Y float32 [M][L]; on the integer tensor
+ * cores, as adx_rsvd_rows_ws. Sums are exact integers: they do not depend on their order. */
 int adx_rsvd_cols(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* Y, int L,
                   int accumulate, float* Z, void* workspace, size_t workspace_bytes,
                   void* stream);

@@ -387,6 +387,195 @@ __global__ void sqp_kernel(const double* __restrict__ H, const double* __restric
   }
 }
 
+// ---------------------------------------------------------------- SQP, K <= 16
+//
+// The same solves with the tableau in registers, for K <= KM <= 16. A row whose active set
+// cycles runs all QP_MAX_ITER iterations, and such rows set the time of a launch (3,800
+// cycles an iteration with the tableau in shared memory, 2.0 ms a launch at any row count;
+// 0.61 ms here), so what counts is the latency of one iteration. Lane i holds row i of the tableau: the
+// parameters' columns, the constraint's (position KM), its last column (the step u_i) and
+// the last row's element i. A sweep on pivot k broadcasts p * tmp through shared memory and
+// is one multiply-add per element; every element sees the operations of sweep() above
+// in the same order, so the results are the same to the last bit.
+template <int KM, bool SIMPLEX>
+struct RegTableau {
+  static constexpr int C = KM + (SIMPLEX ? 1 : 0);   // parameters and the constraint
+  double t[C];      // row `lane`: columns 0..K-1 (zeros to KM), the constraint at KM
+  double last;      // row `lane`, last column
+  double lrow;      // last row, column `lane`
+  double diag;      // t[lane], kept beside it (a register array has no lane index)
+
+  // sweep on pivot position I; pv: C doubles of the warp's shared memory
+  template <int I>
+  __device__ __forceinline__ void sweep_at(bool inverse, int lane, double* pv) {
+    const double piv = __shfl_sync(0xffffffffu, diag, I);
+    if (piv == 0.0) return;
+    const double tmp_last = __shfl_sync(0xffffffffu, lrow, I);   // before the pivot's row and column go to zero
+    const double p = 1.0 / piv;
+    const bool me = lane == I;
+    const double tmp = me ? (inverse ? 1.0 : -1.0) : t[I];
+    const double mine = p * tmp;
+    if (lane < C) pv[lane] = mine;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const double base = i == I ? 0.0 : (me ? 0.0 : t[i]);
+      t[i] = fma(-pv[i], tmp, base);
+    }
+    last = fma(-(p * tmp_last), tmp, me ? 0.0 : last);
+    lrow = fma(-mine, tmp_last, me ? 0.0 : lrow);
+    diag = fma(-mine, tmp, me ? 0.0 : diag);
+    __syncwarp();
+  }
+
+  // the pivot is warp-uniform: a branch to the code of that pivot instead of selecting its
+  // column out of the registers
+  __device__ __forceinline__ void sweep(int k, bool inverse, int lane, double* pv) {
+#define ADX_SWEEP(I) case I: if constexpr (I < C) sweep_at<I>(inverse, lane, pv); break;
+    switch (k) {
+      ADX_SWEEP(0) ADX_SWEEP(1) ADX_SWEEP(2) ADX_SWEEP(3) ADX_SWEEP(4) ADX_SWEEP(5) ADX_SWEEP(6) ADX_SWEEP(7)
+      ADX_SWEEP(8) ADX_SWEEP(9) ADX_SWEEP(10) ADX_SWEEP(11) ADX_SWEEP(12) ADX_SWEEP(13) ADX_SWEEP(14) ADX_SWEEP(15)
+      ADX_SWEEP(16)
+      default: break;
+    }
+#undef ADX_SWEEP
+  }
+};
+
+// quadratic_program() on the register tableau; returns the step of parameter `lane`.
+template <int KM, bool SIMPLEX>
+__device__ __forceinline__ double reg_program(RegTableau<KM, SIMPLEX>& s, int p, double par, int lane, double* pv) {
+  const double small = 1e-5, tol = 1e-8;
+  const bool mine = lane < p;
+  const double diag0 = s.diag;   // each pivot is checked against the diagonal before any sweep
+  double delta = 0.0;
+  for (int i = 0; i < p; ++i) {
+    const double d = __shfl_sync(0xffffffffu, diag0, i), now = __shfl_sync(0xffffffffu, s.diag, i);
+    if (d <= 0.0 || now < d * tol) return delta;
+    s.sweep(i, false, lane, pv);
+  }
+  bool swept = mine;
+  if (SIMPLEX) {
+    if (__shfl_sync(0xffffffffu, s.diag, KM) >= 0.0) return delta;
+    s.sweep(KM, false, lane, pv);
+  }
+  for (int iteration = 1; iteration <= QP_MAX_ITER; ++iteration) {
+    double a = 1.0;
+    const double ui = s.last;
+    if (swept) {
+      const double ai = (ui > 0.0 ? 1.0 : 0.0) - par - delta;
+      if (fabs(ui) > 1e-10) a = fmin(a, ai / ui);
+    }
+    // the parameters' lanes are the first KM: a butterfly within them
+#pragma unroll
+    for (int o = KM > 8 ? 8 : KM > 4 ? 4 : 2; o > 0; o >>= 1) a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
+    if (swept) {
+      delta = delta + a * ui;
+      const double nu = (1.0 - a) * ui;
+      s.last = nu;
+      s.lrow = nu;
+    }
+    const double v = par + delta;
+    const bool critical = (0.0 >= v - small) || (1.0 <= v + small);
+    unsigned m = __ballot_sync(0xffffffffu, swept && fabs(s.diag) > 1e-10 && critical);
+    if (m) {   // the first swept parameter that reached a bound leaves the model
+      const int pick = __ffs(m) - 1;
+      s.sweep(pick, true, lane, pv);
+      if (lane == pick) swept = false;
+      continue;
+    }
+    const bool violation = (s.last > 0.0 && 0.0 >= v - small) || (s.last < 0.0 && 1.0 <= v + small);
+    m = __ballot_sync(0xffffffffu, mine && !swept && violation);
+    if (m) {   // the first unswept parameter whose multiplier points into the interior re-enters
+      const int pick = __ffs(m) - 1;
+      s.sweep(pick, false, lane, pv);
+      if (lane == pick) swept = true;
+      continue;
+    }
+    return delta;
+  }
+  return delta;
+}
+
+template <int KM>
+struct RegScratch {
+  double h[KM * KM];         // the row's Hessian
+  double pv[KM + 2], tmp[KM], out[KM];
+};
+
+template <int KM, bool SIMPLEX>
+__global__ void __launch_bounds__(128) sqp_reg_kernel(const double* __restrict__ H, const double* __restrict__ g,
+                                                      const double* __restrict__ X, const double* __restrict__ v_kk,
+                                                      int64_t rows, int K, double* __restrict__ Xn) {
+  __shared__ RegScratch<KM> scratch[4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  RegScratch<KM>& s = scratch[warp];
+  for (int64_t row = (int64_t)blockIdx.x * 4 + warp; row < rows; row += (int64_t)gridDim.x * 4) {
+    const double* Hr = H + row * K * K;
+    const double* gr = g + row * K;
+    const double* xr = X + row * K;
+    for (int e = lane; e < K * K; e += 32) s.h[e] = Hr[e];
+    __syncwarp();
+    const bool mine = lane < K;
+    double mu = 0.0;
+    if (SIMPLEX) {
+      // mu = 2 max(0, (|t|_1 - 2 |t_0|) / K), t = v_kk (H v_kk[:,0]); sums in index order
+      if (mine) {
+        double t = 0.0;
+        for (int j = 0; j < K; ++j) t += s.h[lane * K + j] * v_kk[j * K];
+        s.tmp[lane] = t;
+      }
+      __syncwarp();
+      if (mine) {
+        double t2 = 0.0;
+        for (int j = 0; j < K; ++j) t2 += v_kk[lane * K + j] * s.tmp[j];
+        s.out[lane] = t2;
+      }
+      __syncwarp();
+      double norm1 = 0.0;
+      for (int i = 0; i < K; ++i) norm1 += fabs(s.out[i]);
+      const double m = 2.0 * ((norm1 - 2.0 * fabs(s.out[0])) / K);
+      mu = m < 0.0 ? 0.0 : m;
+      __syncwarp();
+    }
+    RegTableau<KM, SIMPLEX> tab;
+    const double par = mine ? xr[lane] : 0.0, gl = mine ? gr[lane] : 0.0;
+    if (mine) s.out[lane] = par;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < KM; ++i) tab.t[i] = mine && i < K ? s.h[lane * K + i] + mu : 0.0;
+    tab.last = mine ? -gl : 0.0;
+    tab.lrow = tab.last;
+    if (SIMPLEX) {
+      // the constraint's column is 1 at the parameters, its row likewise; its last column 1 - sum x
+      tab.t[SIMPLEX ? KM : 0] = mine ? 1.0 : 0.0;
+      if (lane == KM) {
+#pragma unroll
+        for (int i = 0; i < KM; ++i) tab.t[i] = i < K ? 1.0 : 0.0;
+        double sx = 0.0;
+        for (int i = 0; i < K; ++i) sx += s.out[i];
+        tab.last = 1.0 - sx;
+        tab.lrow = 1.0 - sx;
+      }
+    }
+    tab.diag = mine ? s.h[lane * K + lane] + mu : 0.0;   // 0 at the constraint
+    const double delta = reg_program<KM, SIMPLEX>(tab, K, par, lane, s.pv);
+    double x = par + delta;
+    if (SIMPLEX) {
+      __syncwarp();
+      if (mine) s.out[lane] = x;
+      __syncwarp();
+      if (lane == 0) project_simplex_row(s.out, K, 1e-5);
+      __syncwarp();
+      if (mine) x = s.out[lane];
+    } else {
+      x = fmin(fmax(x, 1e-5), 1.0 - 1e-5);
+    }
+    if (mine) Xn[row * K + lane] = x;
+    __syncwarp();
+  }
+}
+
 template <typename S>
 static int warps_per_block(size_t fixed) {
   // keep a block's shared memory within 96 KiB, at most 8 warps
@@ -435,6 +624,17 @@ template <bool SIMPLEX>
 static int launch_sqp(const double* H, const double* g, const double* X, const double* v_kk, int64_t rows,
                       int K, double* Xn, void* stream) {
   cudaStream_t st = as_stream(stream);
+  // up to 16 the tableau (K + 2 rows) fits a lane per row and its row in registers
+#define LAUNCH(KM) solve::sqp_reg_kernel<KM, SIMPLEX><<<grid_for(rows, 4), 128, 0, st>>>(H, g, X, v_kk, rows, K, Xn)
+  if (K <= 16) {
+    if (K <= 4) LAUNCH(4);
+    else if (K <= 8) LAUNCH(8);
+    else if (K <= 12) LAUNCH(12);
+    else LAUNCH(16);
+    ADX_LAUNCH_CHECK();
+    return ADX_OK;
+  }
+#undef LAUNCH
 #define LAUNCH(KM)                                                                                      \
   {                                                                                                     \
     const int wpb = solve::warps_per_block<solve::SqpScratch<KM>>(0);                                   \
@@ -442,7 +642,7 @@ static int launch_sqp(const double* H, const double* g, const double* X, const d
     ADX_CUDA_TRY(cudaFuncSetAttribute(solve::sqp_kernel<KM, SIMPLEX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
     solve::sqp_kernel<KM, SIMPLEX><<<grid_for(rows, wpb), 32 * wpb, smem, st>>>(H, g, X, v_kk, rows, K, Xn, wpb); \
   }
-  ADX_KM_SWITCH(K, LAUNCH)
+  if (K <= 32) LAUNCH(32) else LAUNCH(64)
 #undef LAUNCH
   ADX_LAUNCH_CHECK();
   return ADX_OK;

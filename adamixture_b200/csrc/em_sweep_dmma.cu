@@ -128,6 +128,29 @@ __device__ __forceinline__ double weight_b(uint32_t code) {
   return __hiloint2double((int)hi, 0);
 }
 
+// fmin(fmax(x, lo), 1 - lo), lo > 0, by the bit patterns, which order as the values do: the
+// MMAs and the float64 comparisons share a pipe, and it is what bounds the sweep (29.1 -> 27.9
+// ms at N=100,000 x M=50,000, K=10). x comes out of an MMA: a NaN is the positive one and
+// goes to the upper bound where fmax would take it to the lower; the model is lost either way.
+__device__ __forceinline__ double clamp_bits(double x, double lo) {
+  const long long l = __double_as_longlong(lo), h = __double_as_longlong(1.0 - lo);
+  long long b = __double_as_longlong(x);
+  b = b < l ? l : b;
+  b = b > h ? h : b;
+  return __longlong_as_double(b);
+}
+
+// Whether every value lies strictly inside (lo, 1 - lo) by its high word (unsigned: negative
+// values, infinities and NaNs do not): then no clamp is needed.
+template <int N>
+__device__ __forceinline__ bool inside(const double (&x)[N], double lo) {
+  const uint32_t first = (uint32_t)__double2hiint(lo) + 1u, span = (uint32_t)__double2hiint(1.0 - lo) - first;
+  bool in = true;
+#pragma unroll
+  for (int e = 0; e < N; ++e) in = in && ((uint32_t)__double2hiint(x[e]) - first) < span;
+  return in;
+}
+
 // The genotype bytes of SNP rows g and g+8 of the chunk at jc for the thread's 8 samples
 // from s0 (0xFF, all missing, past N); rows past the matrix read its last row (those SNPs
 // are masked as missing by the caller).
@@ -171,21 +194,25 @@ __device__ __forceinline__ double renorm_dm(double x, int& e) {
 }
 
 // The log-likelihood factor h^g (1-h)^(2-g) of 4 entries (1 when missing), h clamped to
-// [1e-10, 1-1e-10], multiplied into the thread's running product.
+// [1e-10, 1-1e-10] (CLAMP = false: the caller has checked that it is), multiplied into the
+// thread's running product.
+template <bool CLAMP>
 __device__ __forceinline__ void ll_factors(const double (&hacc)[4], const uint64_t (&w)[2], int nt, double& prod,
                                            int& ex) {
   double f[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const uint32_t code = (uint32_t)(w[e >> 1] >> (8 * (2 * nt + (e & 1)))) & 3u;
-    const double h = fmin(fmax(hacc[e], LL_CLAMP), 1.0 - LL_CLAMP);
+    const double h = CLAMP ? fmin(fmax(hacc[e], LL_CLAMP), 1.0 - LL_CLAMP) : hacc[e];
     const double om = 1.0 - h;
-    const double x = code == 2u ? h : om;
+    const double x = code >= 2u ? h : om;
     const double y = code == 0u ? om : h;
-    f[e] = code == 3u ? 1.0 : x * y;
+    const double xy = x * y;
+    f[e] = code == 3u ? 1.0 : xy;
   }
   prod *= (f[0] * f[1]) * (f[2] * f[3]);
-  prod = renorm_dm(prod, ex);
+  // 8 factors (at least 1e-160 together) between renormalisations: the product stays normal
+  if (nt & 1) prod = renorm_dm(prod, ex);
 }
 
 // The CTA's log-likelihood partial: each thread's log(prod) + ex ln 2, summed over the warp
@@ -345,13 +372,13 @@ __device__ __forceinline__ void sweep_subtile(const Args& a, const Prob& pr, int
             h_tile(hnext, warp * WS + 8 * (g >> 1) + 2 * (nt + 1) + (g & 1));
           }
           const double (&hacc)[4] = hcur;
-          if constexpr (LL) ll_factors(hacc, w, nt, prod, ex);
+          if constexpr (LL) ll_factors<true>(hacc, w, nt, prod, ex);
           double av[4], bv[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             // element e: SNP row g + 8 (e / 2), local sample 8t + 2nt + e % 2
             const uint32_t code = (uint32_t)(w[e >> 1] >> (8 * (2 * nt + (e & 1)))) & 3u;
-            const double rec = fmin(fmax(hacc[e], E_CLAMP), 1.0 - E_CLAMP);
+            const double rec = clamp_bits(hacc[e], E_CLAMP);
             const double omr = 1.0 - rec;
             // 1/rec and 1/(1-rec) from one reciprocal of x = rec (1 - rec) in [~1e-5, 0.25]:
             // the hardware approximation refined by two Newton-Raphson steps
@@ -607,8 +634,17 @@ __global__ void __launch_bounds__(TPB, 2) loglik_dmma_kernel(Args a, const uint8
           if constexpr (KS & 1)
             mma_f64(hacc[nt], ph[KS - 1][0], ph[KS - 1][1], qt[qrow * QSTR + ((4 * (KS - 1) + t) ^ qsw(qrow))]);
         }
+        // one vote for the chunk's 16 values a thread: the clamps are rarely needed. They and a
+        // renormalisation per 4 factors instead of 8 took 8.08 ms where this takes 6.8 (N=50,000 x
+        // M=100,000, K=8); a vote per tile of 4 was slower than the clamps (8.8 ms)
+        if (__all_sync(0xffffffffu, inside(hacc[0], LL_CLAMP) && inside(hacc[1], LL_CLAMP) &&
+                                        inside(hacc[2], LL_CLAMP) && inside(hacc[3], LL_CLAMP))) {
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) ll_factors(hacc[nt], w, nt, prod, ex);
+          for (int nt = 0; nt < 4; ++nt) ll_factors<false>(hacc[nt], w, nt, prod, ex);
+        } else {
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) ll_factors<true>(hacc[nt], w, nt, prod, ex);
+        }
       }
     }
   }

@@ -36,6 +36,22 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+// The 8 bytes at G + at of a matrix of `total` bytes, at any alignment: three aligned words and a
+// funnel shift. Bytes past the matrix are 0xFF.
+__device__ __forceinline__ uint64_t load8(const uint8_t* __restrict__ G, int64_t total, int64_t at) {
+  const uint8_t* p = G + at;
+  const uint32_t sh = 8u * (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3);
+  const uint8_t* q = p - (sh >> 3);
+  if (q >= G && at + 12 <= total) {
+    const uint32_t w0 = __ldg(reinterpret_cast<const uint32_t*>(q)), w1 = __ldg(reinterpret_cast<const uint32_t*>(q + 4));
+    const uint32_t w2 = __ldg(reinterpret_cast<const uint32_t*>(q + 8));
+    return (uint64_t)__funnelshift_r(w0, w1, sh) | ((uint64_t)__funnelshift_r(w1, w2, sh) << 32);
+  }
+  uint64_t v = 0;
+  for (int b = 0; b < 8; ++b) v |= (uint64_t)(at + b < total ? __ldg(p + b) : (uint8_t)0xFF) << (8 * b);
+  return v;
+}
+
 __device__ __forceinline__ unsigned genotype(uint32_t byte, int s) { return (byte >> (2 * s)) & 3u; }
 
 }  // namespace adx

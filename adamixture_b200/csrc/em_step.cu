@@ -209,15 +209,7 @@ em_sweep_kernel(const uint8_t* __restrict__ G, const R* __restrict__ P, const R*
             }
             return acc;
           };
-          if constexpr (V <= 16) {
-            // at most 16 values: a power-of-two vector of VR, reduced with fewer shuffles
-            constexpr int VR = V <= 4 ? 4 : (V <= 8 ? 8 : 16);
-            R part[VR];
-#pragma unroll
-            for (int v = 0; v < VR; ++v) part[v] = part_of(v);
-            // lanes >= VR hold copies of lanes & (VR - 1): slots V.. of red are never read
-            red[warp][jl][lane] = reduce_scatter_small<VR>(part, lane);
-          } else if constexpr (V < 32 && ((V - 16) & (V - 17)) == 0) {
+          if constexpr (V > 16 && V < 32 && ((V - 16) & (V - 17)) == 0) {
             // 16 + 4 or 16 + 8 values: two power-of-two vectors, 16 + 6 or 16 + 9 shuffle
             // steps instead of 31; lane l < 16 holds value l, lane 16 + i value 16 + i
             constexpr int VR2 = V - 16;
@@ -265,6 +257,250 @@ em_sweep_kernel(const uint8_t* __restrict__ G, const R* __restrict__ P, const R*
     first = false;
   }
 }
+
+// ---------------------------------------------------------------- float32 sweep, K <= 8
+//
+// The float32 sweep for the K whose default arithmetic it is. The same statistics, partition
+// and partials as em_sweep_kernel<float>; what bounds both is instruction issue, so the work
+// per entry is cut: a thread owns 8 consecutive samples and computes them as four packed
+// float32 pairs (h, T, A and B are fma.rn.f32x2: the pairs run along the samples, so every
+// product uses the same packed copy of Q), the 2K sums of a SNP over its 8 samples go to
+// shared memory once per SNP as 16-byte stores, and after a packed quad of SNPs the warp sums
+// them by columns (16-byte loads) -- about 2 instructions an entry where the butterfly over
+// the lanes of 4 samples took 15. The reciprocal of rec (1 - rec) is the hardware
+// approximation (1 ulp) refined by one Newton-Raphson step. N=20,000 x M=100,000, K=6: 5.8 ->
+// 4.0 ms an iteration (36 instructions an entry, 54 % of the packed FMA rate).
+namespace f32s {
+
+constexpr int TPB = 128;
+constexpr int WARPS = TPB / 32;
+constexpr int C = 8;                 // samples per thread
+constexpr int W = TPB * C;           // samples per sub-tile
+constexpr int CH = 32;               // SNP blocks are whole multiples
+
+using u64 = unsigned long long;
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+  u64 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+  u64 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+  u64 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ u64 pack2(float lo, float hi) {
+  u64 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ float rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+template <int K>
+struct Cfg {
+  static constexpr int V = 2 * K;
+  static constexpr int V4 = (V + 3) / 4;                        // 16-byte columns of a SNP's sums
+  static constexpr int RS = V4 == 1 ? 4 : V4 <= 3 ? 12 : 20;    // floats per lane: 16-byte stores free of conflicts
+  static constexpr int SS = 32 * RS + (V4 == 3 ? 12 : 0);       // floats per SNP: column loads likewise (nearly)
+  static constexpr int COLS = 4 * V4;                           // columns of a quad of SNPs
+  static constexpr int LPC = COLS == 4 ? 8 : COLS == 8 ? 4 : 2; // lanes that share a column
+  static constexpr int KP = (K + 1) / 2 * 2;                    // P row of a SNP: pairs {p, p}, 16-byte loads
+  static constexpr int OCC = K <= 2 ? 5 : K <= 4 ? 4 : K <= 6 ? 3 : 2;   // CTAs per SM: registers without spills
+  static constexpr int CHK = K <= 6 ? 32 : 16;                  // SNPs per staged chunk (48 KB of shared memory)
+};
+
+template <int K>
+__global__ void __launch_bounds__(TPB, Cfg<K>::OCC)
+em_sweep_f32_kernel(const uint8_t* __restrict__ G, const float* __restrict__ P, const float* __restrict__ Q, int64_t M,
+                    int64_t N, int64_t n_stile, int n_split, int n_mblk, int64_t mb, float* __restrict__ ABp,
+                    float* __restrict__ Tp) {
+  using F = Cfg<K>;
+  constexpr int CH = F::CHK, V = F::V, V4 = F::V4, RS = F::RS, SS = F::SS, LPC = F::LPC, KP = F::KP;
+  __shared__ __align__(16) u64 Ps[CH][KP];
+  __shared__ __align__(16) float part[WARPS][4 * SS];
+  __shared__ __align__(16) float red[WARPS][CH][4 * V4];
+  const int mblk = blockIdx.x % n_mblk;
+  const int split = blockIdx.x / n_mblk;
+  const int64_t j0 = (int64_t)mblk * mb;
+  const int64_t j1 = min(M, j0 + mb);
+  const int64_t total = ((M + 3) >> 2) * N;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const u64 one2 = pack2(1.0f, 1.0f), mone2 = pack2(-1.0f, -1.0f);
+  const float ELO = (float)E_CLAMP, EHI = (float)(1.0 - E_CLAMP);
+  // weights as the high halves of float32 values by the 2-bit code (low halves 0), two per byte
+  // permute: -g -> {-0, -1, -2, -0} (its product with -1/rec is a), 2 - g -> {2, 1, 0, 0}
+  constexpr uint32_t GA_LO = 0xBF808000u, GA_HI = 0x8000C000u, GB_LO = 0x3F804000u, GB_HI = 0x00000000u;
+
+  bool first = true;
+  for (int64_t st = split; st < n_stile; st += n_split) {
+    const int64_t i0 = st * W + (int64_t)threadIdx.x * C;
+    u64 q[C / 2][K], tt[C / 2][K], tb[C / 2];
+#pragma unroll
+    for (int v = 0; v < C / 2; ++v) {
+      tb[v] = 0ull;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        tt[v][k] = 0ull;
+        q[v][k] = pack2(i0 + 2 * v < N ? Q[(i0 + 2 * v) * K + k] : 0.0f, i0 + 2 * v + 1 < N ? Q[(i0 + 2 * v + 1) * K + k] : 0.0f);
+      }
+    }
+    // the 8 bytes of the thread's samples in the packed row of SNP j. Samples past N read the
+    // next row's (or 0xFF): their Q is zero, so they add nothing, and their T is not written
+    auto bytes_of = [&](int64_t j) -> uint64_t {
+      return i0 < N ? load8(G, total, (j >> 2) * N + i0) : ~0ull;
+    };
+    uint64_t next = bytes_of(j0);
+    // a chunk's P values, loaded a chunk ahead of their use
+    constexpr int PPT = (CH * KP + TPB - 1) / TPB;
+    float pnext[PPT];
+    auto load_p = [&](int64_t c0) {
+#pragma unroll
+      for (int u = 0; u < PPT; ++u) {
+        const int e = threadIdx.x + u * TPB, jl = e / KP, k = e - jl * KP;
+        pnext[u] = e < CH * KP && c0 + jl < j1 && k < K ? P[(c0 + jl) * K + k] : 0.0f;
+      }
+    };
+    load_p(j0);
+    for (int64_t c0 = j0; c0 < j1; c0 += CH) {
+      const int cn = (int)min((int64_t)CH, j1 - c0);
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < PPT; ++u) {
+        const int e = threadIdx.x + u * TPB;
+        if (e < CH * KP) (&Ps[0][0])[e] = pack2(pnext[u], pnext[u]);
+      }
+      __syncthreads();
+      if (c0 + CH < j1) load_p(c0 + CH);
+      for (int qd = 0; qd < cn; qd += 4) {
+        const uint64_t bytes = next;
+        if (c0 + qd + 4 < j1) next = bytes_of(c0 + qd + 4);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const int jl = qd + s;
+          u64 p[KP];
+#pragma unroll
+          for (int k = 0; k < KP; k += 2) {
+            const ulonglong2 pp = *reinterpret_cast<const ulonglong2*>(&Ps[jl][k]);
+            p[k] = pp.x;
+            p[k + 1] = pp.y;
+          }
+          u64 a[C / 2], b[C / 2];
+#pragma unroll
+          for (int v = 0; v < C / 2; ++v) {
+            u64 h = mul2(p[0], q[v][0]);
+#pragma unroll
+            for (int k = 1; k < K; ++k) h = fma2(p[k], q[v][k], h);
+            float h0, h1;
+            unpack2(h, h0, h1);
+            const u64 rec = pack2(fminf(fmaxf(h0, ELO), EHI), fminf(fmaxf(h1, ELO), EHI));
+            const u64 nom = add2(rec, mone2);          // -(1 - rec)
+            const u64 nx = mul2(rec, nom);             // -rec (1 - rec)
+            float x0, x1;
+            unpack2(nx, x0, x1);
+            u64 r = pack2(rcp(-x0), rcp(-x1));
+            r = fma2(r, fma2(nx, r, one2), r);
+            // codes of the two samples (SNPs past the range: missing), then both weights of each
+            uint32_t t2 = (uint32_t)(bytes >> (16 * v + 2 * s)) & 0x0303u;
+            if (jl >= cn) t2 = 0x0303u;
+            const uint32_t sel = t2 * 0x22u + 0x1010u;
+            const uint32_t wa = __byte_perm(GA_LO, GA_HI, sel), wb = __byte_perm(GB_LO, GB_HI, sel);
+            const u64 ga = ((u64)(wa & 0xFFFF0000u) << 32) | (wa << 16), gb = ((u64)(wb & 0xFFFF0000u) << 32) | (wb << 16);
+            a[v] = mul2(ga, mul2(nom, r));
+            b[v] = mul2(gb, mul2(rec, r));
+            tb[v] = add2(tb[v], b[v]);
+            const u64 d = fma2(b[v], mone2, a[v]);
+#pragma unroll
+            for (int k = 0; k < K; ++k) tt[v][k] = fma2(d, p[k], tt[v][k]);
+          }
+          float out[4 * V4];
+#pragma unroll
+          for (int k = 0; k < 4 * V4; ++k) {
+            if (k >= V) { out[k] = 0.0f; continue; }
+            const int kk = k < K ? k : k - K;
+            u64 m = mul2(k < K ? a[0] : b[0], q[0][kk]);
+#pragma unroll
+            for (int v = 1; v < C / 2; ++v) m = fma2(k < K ? a[v] : b[v], q[v][kk], m);
+            float lo, hi;
+            unpack2(m, lo, hi);
+            out[k] = lo + hi;
+          }
+          float4* dst = reinterpret_cast<float4*>(&part[warp][s * SS + lane * RS]);
+#pragma unroll
+          for (int c = 0; c < V4; ++c) dst[c] = make_float4(out[4 * c], out[4 * c + 1], out[4 * c + 2], out[4 * c + 3]);
+        }
+        __syncwarp();
+        // column c = (SNP, 4 sums): LPC lanes add 32 / LPC rows each
+        {
+          const int c = min(lane / LPC, F::COLS - 1), hl = lane % LPC;
+          const int s = c / V4, qq = c - s * V4;
+          const float* src = &part[warp][s * SS + hl * RS + 4 * qq];
+          float4 x = *reinterpret_cast<const float4*>(src);
+          u64 lo = pack2(x.x, x.y), hi = pack2(x.z, x.w);
+#pragma unroll
+          for (int r = 1; r < 32 / LPC; ++r) {
+            const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(src + r * LPC * RS);
+            lo = add2(lo, y.x);
+            hi = add2(hi, y.y);
+          }
+#pragma unroll
+          for (int o = 1; o < LPC; o <<= 1) {
+            lo = add2(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = add2(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+          }
+          if (hl == 0 && lane / LPC < F::COLS)
+            *reinterpret_cast<ulonglong2*>(&red[warp][qd + s][4 * qq]) = make_ulonglong2(lo, hi);
+        }
+        __syncwarp();
+      }
+      __syncthreads();
+      for (int e = threadIdx.x; e < cn * V; e += TPB) {
+        const int jl = e / V, v = e - jl * V;
+        float sum = 0.0f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) sum += red[w][jl][v];
+        // the block is the only writer of the element and this thread always adds it, so an
+        // add in memory keeps the order, and nothing waits for the old value
+        float* dst = ABp + ((int64_t)split * M + (c0 + jl)) * V + v;
+        if (first) *dst = sum;
+        else atomicAdd(dst, sum);
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < C / 2; ++v) {
+      float b0, b1;
+      unpack2(tb[v], b0, b1);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int64_t i = i0 + 2 * v + u;
+        if (i >= N) continue;
+        float* dst = Tp + ((int64_t)mblk * N + i) * K;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          float t0, t1;
+          unpack2(tt[v][k], t0, t1);
+          dst[k] = (u ? t1 : t0) + (u ? b1 : b0);
+        }
+      }
+    }
+    first = false;
+  }
+}
+
+constexpr int MAX_K = 8;
+
+}  // namespace f32s
 
 // ---------------------------------------------------------------- reduce / targets / Adam
 
@@ -447,6 +683,10 @@ int em_plan(int64_t M, int64_t N, int K, int prec, EmPlan& pl) {
     W = dmma_plan_width();
     CH = dmma_plan_chunk();
   }
+  if (prec == ADX_F32 && K <= f32s::MAX_K) {
+    W = f32s::W;
+    CH = f32s::CH;
+  }
   pl.W = W; pl.CH = CH;
   pl.elem_size = prec == ADX_F64 ? sizeof(double) : sizeof(float);
   pl.n_stile = ceil_div(N, W);
@@ -477,10 +717,34 @@ static int launch_sweep(const EmPlan& pl, const uint8_t* G, const void* P, const
   R* ABp = reinterpret_cast<R*>(reinterpret_cast<uint8_t*>(ws) + EmPlan::HEADER);
   R* Tp = ABp + pl.ab_elems;
   const dim3 grid((unsigned)(pl.n_split * pl.n_mblk));
+  if constexpr (sizeof(R) == 4) {
+#define ADX_F32_CASE(KK)                                                                                           \
+  case KK:                                                                                                         \
+    f32s::em_sweep_f32_kernel<KK><<<grid, f32s::TPB, 0, st>>>(G, (const float*)P, (const float*)Q, pl.M, pl.N,       \
+                                                              pl.n_stile, pl.n_split, pl.n_mblk, pl.mb, ABp, Tp);  \
+    ADX_LAUNCH_CHECK();                                                                                            \
+    return ADX_OK;
+    switch (pl.K) {
+      ADX_F32_CASE(1) ADX_F32_CASE(2) ADX_F32_CASE(3) ADX_F32_CASE(4)
+      ADX_F32_CASE(5) ADX_F32_CASE(6) ADX_F32_CASE(7) ADX_F32_CASE(8)
+      default: break;
+    }
+#undef ADX_F32_CASE
+  }
+  // float32 above K = 8, float64 above K = 16 (the float64 MMA form)
 #define LAUNCH(KM)                                                                              \
   em_sweep_kernel<R, KM><<<grid, TPB, 0, st>>>(G, (const R*)P, (const R*)Q, pl.M, pl.N, pl.K,   \
                                                pl.n_stile, pl.n_split, pl.n_mblk, pl.mb, ABp, Tp)
-  ADX_KMAX_SWITCH(pl.kmax, LAUNCH)
+  switch (pl.kmax) {
+    case 10: if constexpr (sizeof(R) == 4) { LAUNCH(10); } break;
+    case 12: if constexpr (sizeof(R) == 4) { LAUNCH(12); } break;
+    case 16: if constexpr (sizeof(R) == 4) { LAUNCH(16); } break;
+    case 24: LAUNCH(24); break;
+    case 32: LAUNCH(32); break;
+    case 48: LAUNCH(48); break;
+    case 64: LAUNCH(64); break;
+    default: break;
+  }
 #undef LAUNCH
   ADX_LAUNCH_CHECK();
   return ADX_OK;

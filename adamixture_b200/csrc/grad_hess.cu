@@ -340,21 +340,6 @@ __device__ __forceinline__ double times_weight(double x, bool zero, bool two) {
   return zero ? 0.0 : __hiloint2double(hi, __double2loint(x));
 }
 
-// The 8 bytes at G + at (rows * N bytes in all); bytes past the matrix are 0xFF.
-__device__ __forceinline__ uint64_t load8(const uint8_t* __restrict__ G, int64_t total, int64_t at) {
-  const uint8_t* p = G + at;
-  const uint32_t sh = 8u * (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3);
-  const uint8_t* q = p - (sh >> 3);
-  if (q >= G && at + 12 <= total) {
-    const uint32_t w0 = __ldg(reinterpret_cast<const uint32_t*>(q)), w1 = __ldg(reinterpret_cast<const uint32_t*>(q + 4));
-    const uint32_t w2 = __ldg(reinterpret_cast<const uint32_t*>(q + 8));
-    return (uint64_t)__funnelshift_r(w0, w1, sh) | ((uint64_t)__funnelshift_r(w1, w2, sh) << 32);
-  }
-  uint64_t v = 0;
-  for (int b = 0; b < 8; ++b) v |= (uint64_t)(at + b < total ? __ldg(p + b) : (uint8_t)0xFF) << (8 * b);
-  return v;
-}
-
 template <bool QSIDE, int K>
 __global__ void __launch_bounds__(32 * MWARPS, Shape<QSIDE, K>::OCC) grad_hess_mma_kernel(Args a) {
   using S = Shape<QSIDE, K>;

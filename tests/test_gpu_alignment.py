@@ -71,3 +71,37 @@ def test_bed_and_statistics_do_not_depend_on_alignment(ops, N, M):
             np.testing.assert_allclose(ops.allele_frequency(P, M).cpu().numpy(), f, rtol=2.0 ** -22, atol=0)
             assert np.array_equal(ops.sample_counts(P, M).cpu().numpy(), 2.0 * seen.sum(0))
             assert np.array_equal(ops.sample_het_counts(P, M).cpu().numpy(), (G == 1).sum(0))
+
+
+def float32_bounds(G, P, Q):
+    """Per-element error bounds of float32 statistics, u = 2^-24: h has K roundings (its terms
+    are positive), 1 - rec inherits h's absolute error, the ratios and weights add a few more
+    roundings, and a sum of n positive terms at most n; T's two parts are bounded by the sum
+    of their magnitudes."""
+    u, K, (M, N) = 2.0 ** -24, P.shape[1], G.shape
+    h = np.clip(P @ Q.T, 1e-5, 1 - 1e-5)
+    seen = G != 3
+    a, b = np.where(seen, G / h, 0.0), np.where(seen, (2.0 - G) / (1 - h), 0.0)
+    ea, eb = a * u * (K + 8), b * u * (K * h / (1 - h) + 8)
+    A = ea @ Q + a @ Q * N * u
+    B = eb @ Q + b @ Q * N * u
+    T = (ea + eb).T @ P + eb.sum(0)[:, None] + ((a + b).T @ P + b.sum(0)[:, None]) * M * u
+    return A, B, T
+
+
+@pytest.mark.parametrize("K", range(1, 9))
+def test_float32_sweep_of_small_k(ops, K):
+    # every K with the packed-pair kernel: samples and SNPs that end inside a thread's 8, a
+    # packed quad and a chunk, several sub-tiles and blocks, any start address
+    for N, M in ((5, 3), (1024, 33), (1025, 64), (2051, 517)):
+        G, P, Q = cohort(N, M, K, K * N + M)
+        packed = orc.pack(G)
+        P32, Q32 = torch.from_numpy(P).float().cuda(), torch.from_numpy(Q).float().cuda()
+        Pd, Qd = P32.double().cpu().numpy(), Q32.double().cpu().numpy()
+        want = orc.em_stats(G, Pd, Qd)[:3]
+        ref = ops.em_stats(placed(packed, 0), P32, Q32, M, "f32")
+        for g, w, tol in zip(ref, want, float32_bounds(G, Pd, Qd)):
+            assert (np.abs(g.cpu().numpy() - w) <= tol).all()
+        for off in (1, 6, 11):
+            got = ops.em_stats(placed(packed, off), P32, Q32, M, "f32")
+            assert all(torch.equal(g, r) for g, r in zip(got, ref)), off

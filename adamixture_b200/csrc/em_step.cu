@@ -512,7 +512,18 @@ struct AdamArgs {
 
 __device__ __forceinline__ double adam_step_no(const AdamArgs& ad) { return ad.t_dev ? *ad.t_dev + ad.t : ad.t; }
 
+// Adds v over the warp's lanes (32 lanes a row) in a fixed order; every lane gets the sum.
+template <int KMAX>
+__device__ __forceinline__ void warp_sum(double (&v)[KMAX]) {
+#pragma unroll
+  for (int k = 0; k < KMAX; ++k)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+}
+
 // mode 0: write A, B, T (float64 statistics). mode 1: EM targets + Adam move on P and Q.
+// gp, gq: threads per P and Q row, 1 or 32. One adds a row's partials in turn; 32 add every
+// 32nd and then each other's. The first p_blocks blocks do the P rows.
 template <typename R, int KMAX>
 __global__ void em_update_kernel(const R* __restrict__ ABp, const R* __restrict__ Tp, int64_t M,
                                  int64_t N, int K, int n_split, int n_mblk, int mode,
@@ -521,22 +532,32 @@ __global__ void em_update_kernel(const R* __restrict__ ABp, const R* __restrict_
                                  double* __restrict__ P, double* __restrict__ Q,
                                  float* __restrict__ P32, float* __restrict__ Q32,
                                  double* __restrict__ mP, double* __restrict__ vP,
-                                 double* __restrict__ mQ, double* __restrict__ vQ, AdamArgs ad) {
-  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= M + N) return;
+                                 double* __restrict__ mQ, double* __restrict__ vQ, AdamArgs ad, unsigned p_blocks,
+                                 int gp, int gq) {
+  const bool p_side = blockIdx.x < p_blocks;
+  const int g = p_side ? gp : gq;
+  const int64_t idx = (int64_t)(p_side ? blockIdx.x : blockIdx.x - p_blocks) * blockDim.x + threadIdx.x;
+  const int64_t row = g == 1 ? idx : idx >> 5;
+  const int part0 = g == 1 ? 0 : (int)(idx & 31);
+  if (row >= (p_side ? M : N)) return;   // whole warps when g = 32
   const double t = adam_step_no(ad);
   const double bc1 = 1.0 - pow(ad.b1, t);
   const double bc2 = 1.0 - pow(ad.b2, t);
-  if (row < M) {
+  if (p_side) {
     const int64_t j = row;
     double A[KMAX], B[KMAX];
 #pragma unroll
     for (int k = 0; k < KMAX; ++k) { A[k] = 0.0; B[k] = 0.0; }
-    for (int s = 0; s < n_split; ++s) {
+    for (int s = part0; s < n_split; s += g) {
       const R* src = ABp + ((int64_t)s * M + j) * (2 * K);
 #pragma unroll
       for (int k = 0; k < KMAX; ++k)
         if (k < K) { A[k] += (double)src[k]; B[k] += (double)src[K + k]; }
+    }
+    if (g > 1) {
+      warp_sum(A);
+      warp_sum(B);
+      if (part0) return;
     }
     if (mode == 0) {
 #pragma unroll
@@ -564,15 +585,19 @@ __global__ void em_update_kernel(const R* __restrict__ ABp, const R* __restrict_
     }
     return;
   }
-  const int64_t i = row - M;
+  const int64_t i = row;
   double T[KMAX];
 #pragma unroll
   for (int k = 0; k < KMAX; ++k) T[k] = 0.0;
-  for (int b = 0; b < n_mblk; ++b) {
+  for (int b = part0; b < n_mblk; b += g) {
     const R* src = Tp + ((int64_t)b * N + i) * K;
 #pragma unroll
     for (int k = 0; k < KMAX; ++k)
       if (k < K) T[k] += (double)src[k];
+  }
+  if (g > 1) {
+    warp_sum(T);
+    if (part0) return;
   }
   if (mode == 0) {
 #pragma unroll
@@ -697,10 +722,31 @@ int em_plan(int64_t M, int64_t N, int K, int prec, EmPlan& pl) {
   n_split = n_split > pl.n_stile ? pl.n_stile : n_split;
   n_split = n_split > PLAN_BLOCKS ? PLAN_BLOCKS : n_split;  // the grid stays within PLAN_BLOCKS
   int64_t max_mblk = ceil_div(M, CH);
-  int64_t n_mblk = PLAN_BLOCKS / n_split;  // the grid stays within PLAN_BLOCKS
-  n_mblk = n_mblk < 1 ? 1 : (n_mblk > max_mblk ? max_mblk : n_mblk);
-  int64_t mb = ceil_div(ceil_div(M, n_mblk), CH) * CH;
-  n_mblk = ceil_div(M, mb);
+  int64_t n_mblk = 0, mb = 0;
+  auto blocks_of = [&](int64_t blocks) {   // the grid stays within `blocks`
+    n_mblk = blocks / n_split;
+    n_mblk = n_mblk < 1 ? 1 : (n_mblk > max_mblk ? max_mblk : n_mblk);
+    mb = ceil_div(ceil_div(M, n_mblk), CH) * CH;
+    n_mblk = ceil_div(M, mb);
+  };
+  blocks_of(PLAN_BLOCKS);
+  // Small cohorts (up to 2,048 samples): with PLAN_BLOCKS a CTA has one or a few chunks of SNPs,
+  // less than what its Q tile, its T partials and the pipeline's start cost (about 4 chunks of the
+  // float64 MMA form, 1 of the float32 pairs). Of 1 to 12 CTAs per SM (148, a constant, as above;
+  // 3 of the float32 form run at a time), the count whose CTAs finish first. At N=105 x M=8,451,
+  // K=7 in float64: 133 CTAs of 4 chunks in one round instead of 529 of one chunk in four.
+  const bool mma64 = prec == ADX_F64 && K <= DMMA_MAX_K, pairs32 = prec == ADX_F32 && K <= f32s::MAX_K;
+  const int64_t own_tiles = ceil_div(pl.n_stile, n_split);
+  if ((mma64 || pairs32) && N <= 2048 && own_tiles * (mb / CH) < 16) {
+    const int64_t slots = mma64 ? 148 : 444, start = mma64 ? 4 : 1;
+    auto rounds = [&]() { return ceil_div(n_split * n_mblk, slots) * own_tiles * (mb / CH + start); };
+    int64_t best = rounds(), best_blocks = PLAN_BLOCKS;
+    for (int64_t blocks = PLAN_BLOCKS / slots * slots; blocks >= slots; blocks -= slots) {
+      blocks_of(blocks);
+      if (rounds() < best) { best = rounds(); best_blocks = blocks; }
+    }
+    blocks_of(best_blocks);
+  }
   pl.n_split = (int)n_split;
   pl.n_mblk = (int)n_mblk;
   pl.mb = mb;
@@ -755,11 +801,18 @@ static int launch_update_from(const EmPlan& pl, const R* ABp, const R* Tp, int m
                               double* T, const double* q_bat, double* P, double* Q, float* P32, float* Q32,
                               double* mP, double* vP, double* mQ, double* vQ, AdamArgs ad, cudaStream_t st) {
   const int threads = 128;
-  const dim3 grid((unsigned)ceil_div(pl.M + pl.N, threads));
+  // A warp per row where one thread's walk over the partials would be the launch's time: few
+  // rows, many partials. One thread per sample took 130 us of a 150 us iteration at N=105 x
+  // M=8,451, K=7 (529 partials), and 2.70 -> 2.64 ms at N=10,007 (224 partials); at N=20,000 (136
+  // partials) the threads' neighbouring rows make up for it: 3.97 against 4.02 ms.
+  const int gp = pl.M < 16384 && pl.n_split >= 32 ? 32 : 1;
+  const int gq = pl.N < 16384 && pl.n_mblk >= 32 ? 32 : 1;
+  const unsigned p_blocks = (unsigned)ceil_div(pl.M * gp, threads);
+  const dim3 grid(p_blocks + (unsigned)ceil_div(pl.N * gq, threads));
 #define LAUNCH(KM)                                                                          \
   em_update_kernel<R, KM><<<grid, threads, 0, st>>>(ABp, Tp, pl.M, pl.N, pl.K, pl.n_split,  \
                                                     pl.n_mblk, mode, A, B, T, q_bat, P, Q,  \
-                                                    P32, Q32, mP, vP, mQ, vQ, ad)
+                                                    P32, Q32, mP, vP, mQ, vQ, ad, p_blocks, gp, gq)
   ADX_KMAX_SWITCH(pl.kmax, LAUNCH)
 #undef LAUNCH
   ADX_LAUNCH_CHECK();

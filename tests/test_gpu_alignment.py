@@ -105,3 +105,17 @@ def test_float32_sweep_of_small_k(ops, K):
         for off in (1, 6, 11):
             got = ops.em_stats(placed(packed, off), P32, Q32, M, "f32")
             assert all(torch.equal(g, r) for g, r in zip(got, ref)), off
+
+
+@pytest.mark.parametrize("N,M,K", [(20_000, 48, 5), (30_001, 130, 16), (105, 8451, 7), (2048, 1300, 3), (1, 900, 2)])
+def test_partials_of_few_rows(ops, N, M, K):
+    # many partials for few P rows (wide, short matrices) or few Q rows: 32 threads a row, and the
+    # small cohorts' partition. Float64 statistics: a sum of n positive terms is within n 2^-53
+    # of the exact one, its terms within a few roundings and h's K 2^-53 over 1 - h
+    G, P, Q = cohort(N, M, K, N + M)
+    P, Q = np.clip(P, 0.01, 0.99), Q / Q.sum(1, keepdims=True)
+    want = orc.em_stats(G, P, Q)[:3]
+    got = ops.em_stats(placed(orc.pack(G), 0), torch.from_numpy(P).cuda(), torch.from_numpy(Q).cuda(), M, "f64")
+    for g, w, n in zip(got, want, (N, N, 2 * M)):
+        tol = (n + 100 * (K + 8)) * 2.0 ** -53
+        np.testing.assert_allclose(g.cpu().numpy(), w, rtol=tol, atol=100 * tol)

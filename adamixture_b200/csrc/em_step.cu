@@ -269,7 +269,7 @@ em_sweep_kernel(const uint8_t* __restrict__ G, const R* __restrict__ P, const R*
 // them by columns (16-byte loads) -- about 2 instructions an entry where the butterfly over
 // the lanes of 4 samples took 15. The reciprocal of rec (1 - rec) is the hardware
 // approximation (1 ulp) refined by one Newton-Raphson step. N=20,000 x M=100,000, K=6: 5.8 ->
-// 4.0 ms an iteration (36 instructions an entry, 54 % of the packed FMA rate).
+// 3.8 ms an iteration (36 instructions an entry, 54 % of the packed FMA rate).
 namespace f32s {
 
 constexpr int TPB = 128;
@@ -358,10 +358,8 @@ em_sweep_f32_kernel(const uint8_t* __restrict__ G, const float* __restrict__ P, 
     }
     // the 8 bytes of the thread's samples in the packed row of SNP j. Samples past N read the
     // next row's (or 0xFF): their Q is zero, so they add nothing, and their T is not written
-    auto bytes_of = [&](int64_t j) -> uint64_t {
-      return i0 < N ? load8(G, total, (j >> 2) * N + i0) : ~0ull;
-    };
-    uint64_t next = bytes_of(j0);
+    auto fetch = [&](int64_t j) { return i0 < N ? fetch8(G, total, (j >> 2) * N + i0) : Words8{~0u, ~0u, ~0u, 0u}; };
+    Words8 next = fetch(j0);
     // a chunk's P values, loaded a chunk ahead of their use
     constexpr int PPT = (CH * KP + TPB - 1) / TPB;
     float pnext[PPT];
@@ -384,8 +382,8 @@ em_sweep_f32_kernel(const uint8_t* __restrict__ G, const float* __restrict__ P, 
       __syncthreads();
       if (c0 + CH < j1) load_p(c0 + CH);
       for (int qd = 0; qd < cn; qd += 4) {
-        const uint64_t bytes = next;
-        if (c0 + qd + 4 < j1) next = bytes_of(c0 + qd + 4);
+        const uint64_t bytes = next.bytes();
+        if (c0 + qd + 4 < j1) next = fetch(c0 + qd + 4);
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
           const int jl = qd + s;

@@ -27,7 +27,7 @@
 // shared memory and no barrier stands between the two contractions.
 // Reduced entry 8t + 2nt + e of a chunk is column 2t + e of h tile nt: a thread's 8 entries of a row
 // are 8 consecutive genotypes (two packed bytes on the Q side, 8 bytes on the P side).
-// Measured at N=20,000 x M=50,000, K=10: Q side 17.4 -> 11.5 ms, P side 12.4 -> 7.4 ms; at
+// Measured at N=20,000 x M=50,000, K=10: Q side 17.4 -> 11.4 ms, P side 12.4 -> 7.2 ms; at
 // N=2,504 x M=100,003, K=7: 3.8 -> 1.9 and 2.8 -> 1.2 ms (before: 64-row x 64-pair tiles with the
 // coefficients staged in shared memory, K = 7's 28 pairs padded to 64).
 //
@@ -381,26 +381,32 @@ __global__ void __launch_bounds__(32 * MWARPS, Shape<QSIDE, K>::OCC) grad_hess_m
       own[ks][r] = row < n_rows && k < K ? ownF[row * K + k] : 0.0;
     }
 
-  // the 2-bit codes of the thread's 8 reduced entries of rows g and g + 8 of a chunk, 8 bits
-  // apart; 3 (missing) past the reduced axis
-  auto load_codes = [&](int64_t red0, uint64_t (&w)[2]) {
+  // The 2-bit codes of the thread's 8 reduced entries of rows g and g + 8 of a chunk: two packed
+  // bytes on the Q side, 8 bytes on the P side. Loaded a chunk ahead, put together at use; rows
+  // and entries outside the matrix are 3 (missing) or are masked by the caller.
+  struct Codes {
+    Words8 p[QSIDE ? 1 : 2];
+    uint32_t q[2][2];
+  };
+  auto load_codes = [&](int64_t red0, Codes& c) {
     const int64_t first = red0 + 8 * t;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int64_t row = row0 + g + 8 * r;
-      uint64_t v = ~0ull;
       if constexpr (QSIDE) {
-        uint32_t by = 0xFFFFu;
-        if (row < a.N) {
-          const int64_t pr = first >> 2;   // first is a multiple of 8
-          if (pr < prows) by = (by & 0xFF00u) | (uint32_t)__ldg(a.G + pr * a.N + row);
-          if (pr + 1 < prows) by = (by & 0x00FFu) | ((uint32_t)__ldg(a.G + (pr + 1) * a.N + row) << 8);
-        }
-        v = by;
-      } else if (row < a.M && first < n_red) {
-        v = load8(a.G, prows * a.N, (row >> 2) * a.N + first) >> (2 * (uint32_t)(row & 3));
+        const int64_t pr = first >> 2;   // first is a multiple of 8
+        c.q[r][0] = row < a.N && pr < prows ? (uint32_t)__ldg(a.G + pr * a.N + row) : 0xFFu;
+        c.q[r][1] = row < a.N && pr + 1 < prows ? (uint32_t)__ldg(a.G + (pr + 1) * a.N + row) : 0xFFu;
+      } else {
+        c.p[r] = row < a.M && first < n_red ? fetch8(a.G, prows * a.N, (row >> 2) * a.N + first) : Words8{~0u, ~0u, ~0u, 0u};
       }
-      w[r] = v;
+    }
+  };
+  auto codes_of = [&](const Codes& c, uint64_t (&w)[2]) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      if constexpr (QSIDE) w[r] = c.q[r][0] | (c.q[r][1] << 8);
+      else w[r] = c.p[r].bytes() >> (2 * (uint32_t)((row0 + g + 8 * r) & 3));
     }
   };
   auto code_of = [&](uint64_t w, int idx) -> uint32_t {
@@ -424,7 +430,7 @@ __global__ void __launch_bounds__(32 * MWARPS, Shape<QSIDE, K>::OCC) grad_hess_m
   // the axis) are loaded a chunk ahead of their use
   constexpr bool AHEAD = NP <= 5 || NP >= 8;
   constexpr int FPT = (CJ * K + 32 * MWARPS - 1) / (32 * MWARPS);
-  uint64_t next[2];
+  Codes next;
   double fnext[FPT];
   auto load_factors = [&](int64_t red0) {
 #pragma unroll
@@ -437,7 +443,8 @@ __global__ void __launch_bounds__(32 * MWARPS, Shape<QSIDE, K>::OCC) grad_hess_m
   if (AHEAD) load_factors(ch0 * CJ);
   for (int64_t ch = ch0; ch < ch1; ++ch) {
     const int64_t red0 = ch * CJ;
-    uint64_t w[2] = {next[0], next[1]};
+    uint64_t w[2];
+    codes_of(next, w);
     if (!AHEAD) load_factors(red0);
     __syncthreads();   // the previous chunk's readers are done
 #pragma unroll

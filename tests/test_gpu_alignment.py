@@ -119,3 +119,24 @@ def test_partials_of_few_rows(ops, N, M, K):
     for g, w, n in zip(got, want, (N, N, 2 * M)):
         tol = (n + 100 * (K + 8)) * 2.0 ** -53
         np.testing.assert_allclose(g.cpu().numpy(), w, rtol=tol, atol=100 * tol)
+
+
+@pytest.mark.parametrize("K", [1, 2, 5, 8, 10, 11, 16])
+def test_float32_loglik_of_small_k(ops, K):
+    # the packed-pair form: ragged samples, quads and chunks, exponents moved every 4 quads, any
+    # start address. h has K roundings of 2^-24 and 1 - h inherits them; a pair of factors
+    # rounds three times more
+    for N, M in ((1, 1), (9, 35), (1025, 70), (2050, 517)):
+        G, P, Q = cohort(N, M, K, K + N * M)
+        packed = orc.pack(G)
+        P32, Q32 = torch.from_numpy(P).float().cuda(), torch.from_numpy(Q).float().cuda()
+        Pd, Qd = P32.double().cpu().numpy(), Q32.double().cpu().numpy()
+        h = np.clip(Pd @ Qd.T, 1e-10, 1 - 1e-10)
+        seen = G != 3
+        g = np.where(seen, G, 0).astype(float)
+        L = np.where(seen, g * np.log(h) + (2 - g) * np.log1p(-h), 0.0).sum()
+        tol = 2.0 ** -24 * np.where(seen, g * K + (2 - g) * (K * h / (1 - h) + 1) + 2, 0.0).sum() + 1e-12 * abs(L)
+        ref = ops.loglik_device(placed(packed, 0), P32, Q32, M, "f32")
+        assert abs(float(ref) - L) <= tol
+        for off in (1, 6, 15):
+            assert torch.equal(ops.loglik_device(placed(packed, off), P32, Q32, M, "f32"), ref), off

@@ -25,30 +25,40 @@
 // after the last sample tile, A_r/B_r go to the A/B partials of the CTA's split.
 //
 // Warp specialisation: HALF_WGS warpgroups form the ratios of the first 64 samples of every
-// step and as many those of the second 64 (each warpgroup a block of WG_COLS samples); the
-// last warp is the producer. Its lane 0 issues every MMA from precomputed shared-memory
-// descriptors (a step's 34 MMAs cost one 64-bit add per operand), and the warp streams the
-// G tiles (a ring of NG stages, NG-1 steps ahead) and the converted Q tiles (NQ buffers, one
-// sample tile ahead) into shared memory with cp.async. H/Hc live in two TMEM buffers (one
-// per half) and the a/b tiles in two shared-memory buffers (one per step parity), so while
-// one half's warpgroups form their ratios the tensor pipe runs the other half's H and the
-// A/B/T MMAs of the previous step. There is no block-wide barrier in the loop: the warps
-// meet only at mbarriers, and loop counters advance incrementally (no division).
+// step and as many those of the second 64 (each warpgroup a block of WG_COLS samples). One
+// warp streams the G tiles (a ring of NG stages) and the converted Q tiles (NQ buffers) into
+// shared memory with cp.async. Three warps issue the MMAs from precomputed shared-memory
+// descriptors (one 64-bit add per operand): H, A/B and T. H/Hc live in two TMEM buffers (one per
+// half) and the a/b tiles in two shared-memory buffers (one per step parity), so while the
+// warpgroups form the ratios of a step the tensor pipe runs the next step's H and the A/B/T
+// MMAs of the previous one. There is no block-wide barrier in the loop: the warps meet only at
+// mbarriers, and loop counters advance incrementally (no division).
 //
 // TMEM (512 columns, one CTA per SM): H/Hc buffer b at [128b, 128b+128) (H first 64, Hc
-// last 64) | T [256,272) | A_r,B_r [272+32r, 304+32r) for r < 7.
+// last 64) | T [256,272) and [496,512) (even and odd sample tiles) | A_r,B_r [272+32r, 304+32r)
+// for r < 7.
 // Shared-memory operands use the no-swizzle canonical layout (8-row x 16-byte core
 // matrices). One copy of each tile serves both of its MMA views: P_r is the K-major A of H
 // and the MN-major B of T; Q_s is the K-major B of H and the MN-major B of A/B; the a/b
 // tiles are the K-major A of A/B and the MN-major A of T.
 //
-// Synchronisation (mbarriers): hfull[h] (tcgen05.commit: H of half h's next half-step and
-// every MMA issued before it are done), abready[h] (128*HALF_WGS arrivals: half h's
-// warpgroups wrote their a/b columns and finished reading their H buffer), gfull[g] and
-// qfull[q] (32 cp.async arrivals: G stage g / Q buffer q is loaded). Every wait is bounded
-// and also watches a shared abort word; on a timeout the kernel records ADX_ERR_TIMEOUT in
-// the status word, all warps leave their loops, it waits (bounded) for its MMAs in flight,
-// frees its TMEM and returns.
+// Synchronisation (mbarriers): hfull (tcgen05.commit: a step's H is done), hfree (an arrival
+// per consumer warp: it holds its H in registers, the buffers are free), abready[step parity]
+// (an arrival per consumer warp: its a/b columns are written; two barriers, so that no phase can
+// pass unseen by an issuer that is a step behind), abfree[step parity] (two commits: the step's
+// A/B and T are done), gfull[g] and qfull[q] (32 cp.async arrivals: G stage g / Q buffer q is
+// loaded), gfree[g] (an arrival per consumer warp) and qfree[q] (a commit). The consumers take
+// their whole block of H at once and free the buffer before the arithmetic, so the next step's
+// H is there when they come back for it. T has two buffers and is read two steps later, when
+// abfree says that its last batch is done.
+//
+// Measured at N=200,000 x M=500,000, K=10: 75.1 ms (330 GB/s of algorithmic bytes, 106
+// TFLOP/s). One warp that loaded and issued everything took 113.9 ms: an MMA here (M=128, N=16)
+// runs for about 100 cycles beside the consumers, its issuer is held for as long, and each
+// wait of the issuer drained the pipe for some 450 cycles, 5,200 cycles a step in all.
+// Every wait is bounded and also watches a shared abort word; on a timeout the kernel
+// records ADX_ERR_TIMEOUT in the status word, all warps leave their loops, it waits (bounded)
+// for its MMAs in flight, frees its TMEM and returns.
 #include <algorithm>
 #include <functional>
 #include <queue>
@@ -71,8 +81,8 @@ constexpr int HALF = TILE / 2;                          // samples per half-step
 constexpr int HALF_WGS = ADX_TC_HALF_WGS;               // consumer warpgroups per half
 constexpr int WG_COLS = HALF / HALF_WGS;                // samples per warpgroup and half-step
 constexpr int CONSUMER_WARPS = 2 * 4 * HALF_WGS;
-constexpr int PRODUCER_WARP = CONSUMER_WARPS;
-constexpr int TPB = CONSUMER_WARPS * 32 + 32;
+constexpr int LOAD_WARP = CONSUMER_WARPS, H_WARP = LOAD_WARP + 1, AB_WARP = LOAD_WARP + 2, T_WARP = LOAD_WARP + 3;
+constexpr int TPB = CONSUMER_WARPS * 32 + 128;
 constexpr int NG = 4;          // G stages
 constexpr int NQ = 3;          // Q buffers
 static_assert(WG_COLS % 16 == 0, "warpgroup column blocks are whole 16-column TMEM loads");
@@ -88,7 +98,7 @@ constexpr int OFF_G = OFF_Q + NQ * P_TILE_BYTES;        // NG stages
 constexpr int OFF_A = OFF_G + NG * G_TILE_BYTES;        // 2 buffers
 constexpr int OFF_B = OFF_A + 2 * AB_TILE_BYTES;        // 2 buffers
 constexpr int OFF_BAR = OFF_B + 2 * AB_TILE_BYTES;      // mbarriers
-constexpr int N_BARS = 2 + 2 + NG + NQ;
+constexpr int N_BARS = 9 + 2 * NG + 2 * NQ;
 constexpr int OFF_TMEM = OFF_BAR + 8 * N_BARS;          // TMEM address, then the abort word
 constexpr int SMEM_BYTES = OFF_TMEM + 16;
 constexpr int SMEM_ALLOC = SMEM_BYTES + 1024;           // room to align the base to 1024
@@ -99,7 +109,8 @@ static_assert(OFF_G % 16 == 0 && G_TILE_BYTES % 16 == 0 && G_ROW % 16 == 0, "cp.
 static_assert(SMEM_ALLOC < 256 * 1024, "descriptor start field");
 
 // TMEM columns
-constexpr uint32_t COL_T = 256, COL_AB = 272;
+constexpr uint32_t COL_AB = 272;
+__device__ __forceinline__ uint32_t col_t(int sidx) { return (sidx & 1) ? 496u : 256u; }  // T of the CTA's sample tile sidx
 
 // ---------------------------------------------------------------- descriptors
 
@@ -253,7 +264,7 @@ __global__ void q_to_tiles_kernel(const float* __restrict__ Q, int64_t N, int K,
 // (they cover the 128 samples at any offset); the consumers apply the offset, which is a
 // constant of the row within the tile (row_offset). A sample count that is not a multiple of
 // 16 is what real cohorts have: loading such rows byte by byte through one warp took 14.9 ms
-// where these chunks take 2.7 ms (N=10,007 x M=200,003, K=8), the aligned shape's time.
+// where these chunks take the aligned shape's time (2.7 ms then, 1.9 ms now; N=10,007 x M=200,003, K=8).
 // Chunks that would leave the matrix (the last row or two) take byte loads; bytes past the
 // matrix are 0xFF (missing). Samples past N read the next row's bytes or 0xFF: their Q rows
 // are zero, so they add nothing to A and B, and their T is not written. Rows past the matrix
@@ -319,10 +330,18 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sm + OFF_TMEM);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_TMEM + 4);
   const uint32_t bars = smem_u32(sm + OFF_BAR);
-  auto HFULL = [&](int h) { return bars + 8u * (uint32_t)h; };
-  auto ABREADY = [&](int h) { return bars + 16u + 8u * (uint32_t)h; };
-  auto GFULL = [&](int g) { return bars + 32u + 8u * (uint32_t)g; };
-  auto QFULL = [&](int q) { return bars + 32u + 8u * (uint32_t)NG + 8u * (uint32_t)q; };
+  const uint32_t HFULL = bars, HFREE = bars + 8u;
+  auto ABREADY = [&](int st) { return bars + 16u + 8u * (uint32_t)(st & 1); };
+  auto ABFREE = [&](int st) { return bars + 32u + 8u * (uint32_t)(st & 1); };
+  auto GFULL = [&](int g) { return bars + 48u + 8u * (uint32_t)g; };
+  auto GFREE = [&](int g) { return bars + 48u + 8u * (uint32_t)(NG + g); };
+  auto QFULL = [&](int q) { return bars + 48u + 8u * (uint32_t)(2 * NG + q); };
+  auto QFREE = [&](int q) { return bars + 48u + 8u * (uint32_t)(2 * NG + NQ + q); };
+  auto DRAIN = [&](int w) { return bars + 48u + 8u * (uint32_t)(2 * NG + 2 * NQ + w - H_WARP); };
+  // all lanes of a warp leave a wait with the same answer
+  auto warp_wait = [](uint32_t bar, uint32_t parity, volatile int* flag) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, flag));
+  };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   const int mblk = blockIdx.x % a.n_mblk;
@@ -333,19 +352,28 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
   const int n_my = (int)((a.n_stile - split + a.n_split - 1) / a.n_split);  // sample tiles of this CTA
   const int nsteps = n_my * r_eff;
 
-  // ---- prologue: TMEM (producer warp), barriers, P tiles (all threads)
-  if (warp == PRODUCER_WARP) {
+  // ---- prologue: TMEM (H warp), barriers, P tiles (all threads)
+  if (warp == H_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_holder)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
     *abort_flag = 0;
-    for (int h = 0; h < 2; ++h) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(HFULL(h)));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ABREADY(h)), "r"(128 * HALF_WGS));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(HFULL));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(HFREE), "r"(CONSUMER_WARPS));
+    for (int b = 0; b < 2; ++b) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ABREADY(b)), "r"(CONSUMER_WARPS));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(ABFREE(b)));   // A/B and T
     }
-    for (int g = 0; g < NG; ++g) asm volatile("mbarrier.init.shared::cta.b64 [%0], 32;" ::"r"(GFULL(g)));
-    for (int q = 0; q < NQ; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 32;" ::"r"(QFULL(q)));
+    for (int w = H_WARP; w <= T_WARP; ++w) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(DRAIN(w)));
+    for (int g = 0; g < NG; ++g) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 32;" ::"r"(GFULL(g)));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(GFREE(g)), "r"(CONSUMER_WARPS));
+    }
+    for (int q = 0; q < NQ; ++q) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 32;" ::"r"(QFULL(q)));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(QFREE(q)));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   for (int e = tid; e < r_eff * TILE * 2; e += TPB) {
@@ -383,37 +411,45 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
   const uint64_t dPM = sdesc(s_p, 256, 128);    // P_r MN-major (B of T): + 512 r + 32 ks; 1-P: + 256
   constexpr uint64_t B_OFF = (uint64_t)(OFF_B - OFF_A) >> 4;
 
-  // H/Hc of half h of a step on SNP tile r and Q buffer qb, into TMEM buffer h
-  auto issue_h = [&](int r, int qb, int h) {
-    const uint64_t bq = dQK + (uint64_t)(qb * 256 + h * 128);
+  // H/Hc of both halves of a step on SNP tile r and Q buffer qb
+  auto issue_h = [&](int r, int qb) {
     const uint64_t ap = dPK + (uint64_t)(r * 512);
-    const uint32_t col = tmem + (uint32_t)h * 128;
-    mma_f16kind(col, ap, bq, ID_H, 0);
-    mma_f16kind(col + HALF, ap + 256, bq, ID_H, 0);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint64_t bq = dQK + (uint64_t)(qb * 256 + h * 128);
+      const uint32_t col = tmem + (uint32_t)h * 128;
+      mma_f16kind(col, ap, bq, ID_H, 0);
+      mma_f16kind(col + HALF, ap + 256, bq, ID_H, 0);
+    }
   };
-  // A/B/T MMAs of a step on SNP tile r, Q buffer qb, a/b buffer buf
-  auto issue_abt = [&](int r, int qb, int buf, bool acc_ab) {
+  // A/B MMAs of a step on SNP tile r, Q buffer qb, a/b buffer buf, of the CTA's sample tile sidx
+  auto issue_ab = [&](int r, int qb, int buf, int sidx) {
     const uint64_t qm = dQM + (uint64_t)(qb * 256);
     const uint64_t ak = dAK + (uint64_t)(buf * 2048);
     const uint32_t tab = tmem + COL_AB + 32u * (uint32_t)r;
 #pragma unroll
     for (int ks = 0; ks < TILE / 16; ++ks) {
-      const uint32_t acc = (acc_ab || ks > 0) ? 1u : 0u;
+      const uint32_t acc = (sidx > 0 || ks > 0) ? 1u : 0u;
       mma_f16kind(tab, ak + 16 * ks, qm + 32 * ks, ID_AB, acc);
       mma_f16kind(tab + 16, ak + B_OFF + 16 * ks, qm + 32 * ks, ID_AB, acc);
     }
+  };
+  // its T MMAs
+  auto issue_t = [&](int r, int buf, int sidx) {
+    const uint32_t tt = tmem + col_t(sidx);
     const uint64_t am = dAM + (uint64_t)(buf * 2048);
     const uint64_t pm = dPM + (uint64_t)(r * 512);
 #pragma unroll
     for (int ks = 0; ks < TILE / 16; ++ks) {
       const uint32_t acc = (r > 0 || ks > 0) ? 1u : 0u;
-      mma_f16kind(tmem + COL_T, am + 256 * ks, pm + 32 * ks, ID_T, acc);
-      mma_f16kind(tmem + COL_T, am + B_OFF + 256 * ks, pm + 256 + 32 * ks, ID_T, 1u);
+      mma_f16kind(tt, am + 256 * ks, pm + 32 * ks, ID_T, acc);
+      mma_f16kind(tt, am + B_OFF + 256 * ks, pm + 256 + 32 * ks, ID_T, 1u);
     }
   };
-  auto write_t = [&](int64_t s) {  // one warpgroup: T rows (samples) of sample tile s
+  auto write_t = [&](int sidx) {  // one warpgroup: T rows (samples) of the CTA's sample tile sidx
+    const int64_t s = s_first + (int64_t)sidx * a.n_split;
     uint32_t v[16];
-    tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + COL_T, v);
+    tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + col_t(sidx), v);
     tmem_wait_ld();
     const int64_t i = s * TILE + (warp & 3) * 32 + lane;
     if (i < a.N) {
@@ -425,86 +461,69 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
   };
 
   bool aborted = false;
-  if (warp == PRODUCER_WARP) {
-    // ---------------------------------------------------------------- producer
-    // Q of sample tile t goes to buffer t % NQ (k-th fill: parity k & 1), G of step g to
-    // stage g % NG; both are tracked by counters.
-    producer_load_q(a, s_first, sm + OFF_Q, QFULL(0));
-    if (n_my > 1) producer_load_q(a, s_first + a.n_split, sm + OFF_Q + P_TILE_BYTES, QFULL(1));
-    int gst = 0, gr = 0, gsidx = 0, gstage = 0;  // next G load: step, SNP tile, sample tile, stage
-    auto load_next_g = [&]() {
-      producer_load_g<AL>(a, (jb + (int64_t)gr * TILE) >> 2, (s_first + (int64_t)gsidx * a.n_split) * TILE,
+  if (warp == LOAD_WARP) {
+    // ---------------------------------------------------------------- loads
+    // G of step m goes to stage m % NG; with the first step of the CTA's sample tile t, its Q tile
+    // goes to buffer t % NQ. Both wait for the previous fill's readers.
+    int mr = 0, t = 0, gstage = 0, qbuf = 0;
+    uint32_t gfill = 0, qfill = 0;
+    for (int m = 0; m < nsteps; ++m) {
+      if (mr == 0) {
+        if (qfill > 0 && !warp_wait(QFREE(qbuf), (qfill - 1) & 1u, abort_flag)) { aborted = true; break; }
+        producer_load_q(a, s_first + (int64_t)t * a.n_split, sm + OFF_Q + qbuf * P_TILE_BYTES, QFULL(qbuf));
+        if (++qbuf == NQ) { qbuf = 0; ++qfill; }
+      }
+      if (gfill > 0 && !warp_wait(GFREE(gstage), (gfill - 1) & 1u, abort_flag)) { aborted = true; break; }
+      producer_load_g<AL>(a, (jb + (int64_t)mr * TILE) >> 2, (s_first + (int64_t)t * a.n_split) * TILE,
                           sm + OFF_G + gstage * G_TILE_BYTES, GFULL(gstage));
-      ++gst;
-      if (++gr == r_eff) { gr = 0; ++gsidx; }
-      if (++gstage == NG) gstage = 0;
-    };
-    while (gst < NG - 1 && gst < nsteps) load_next_g();
-    if (!mbar_wait(QFULL(0), 0u, abort_flag)) aborted = true;
-    fence_async_smem();
-    if (!aborted && lane == 0) {
-      issue_h(0, 0, 0);
-      mma_commit(HFULL(0));
-      issue_h(0, 0, 1);
-      mma_commit(HFULL(1));
+      if (++mr == r_eff) { mr = 0; ++t; }
+      if (++gstage == NG) { gstage = 0; ++gfill; }
     }
-    __syncwarp();
-    int r = 0, sidx = 0, qb = 0;       // the current step's SNP tile, sample tile, Q buffer
-    uint32_t qpar = 0u;                // parity of the Q buffer's fill for sample tile sidx
-    uint32_t pab0 = 0u, pab1 = 0u;
-    for (int st = 0; st < nsteps && !aborted; ++st) {
-      int r1 = r + 1, sidx1 = sidx, qb1 = qb;
-      uint32_t qpar1 = qpar;
-      if (r1 == r_eff) {
-        r1 = 0;
-        ++sidx1;
-        if (++qb1 == NQ) { qb1 = 0; qpar1 ^= 1u; }
-      }
-      const bool more = st + 1 < nsteps;
-      // ---- half 0 of step st is formed: refill H buffer 0 with the next step's half 0
-      if (!mbar_wait(ABREADY(0), pab0, abort_flag)) { aborted = true; break; }
-      pab0 ^= 1u;
-      fence_after();
-      // at the first step of sample tile sidx >= 1, prefetch tile sidx + 1 into the buffer
-      // of tile sidx - 2, whose MMAs completed before this barrier phase
-      if (r == 0 && sidx >= 1 && sidx + 1 < n_my) {
-        const int qn = qb + 1 == NQ ? 0 : qb + 1;
-        producer_load_q(a, s_first + (int64_t)(sidx + 1) * a.n_split, sm + OFF_Q + qn * P_TILE_BYTES, QFULL(qn));
-      }
-      if (more && r1 == 0) {  // the next step starts a sample tile: its Q must have landed
-        if (!mbar_wait(QFULL(qb1), qpar1, abort_flag)) { aborted = true; break; }
-        fence_async_smem();
-      }
-      if (lane == 0) {
-        if (more) issue_h(r1, qb1, 0);
-        mma_commit(HFULL(0));
-      }
-      __syncwarp();
-      if (gst < nsteps) load_next_g();  // step st + NG - 1 into the stage step st - 1 used
-      // ---- half 1 of step st is formed: A/B/T of step st, then the next step's half 1
-      if (!mbar_wait(ABREADY(1), pab1, abort_flag)) { aborted = true; break; }
-      pab1 ^= 1u;
-      fence_after();
-      // The next half-1 H goes ahead of this step's A/B/T batch in the (in-order) tensor pipe
-      // and is committed first, so the half-1 warpgroups do not wait for the batch. Where
-      // the next step starts a sample tile the commit follows the batch instead: those
-      // warpgroups read T out of tensor memory after it, so it must cover the tile's last
-      // T MMAs. (The batch's a/b buffer is rewritten two steps later, after commits that
-      // cover it; the last step's commit covers everything.)
-      if (lane == 0) {
-        if (more && r1 != 0) {
-          issue_h(r1, qb1, 1);
-          mma_commit(HFULL(1));
-          issue_abt(r, qb, st & 1, sidx > 0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (warp >= H_WARP) {
+    // ---------------------------------------------------------------- MMAs
+    // Three warps issue: H, A/B and T, each from one lane (an accumulator's MMAs come from one
+    // thread, which keeps their order). The issue of a batch holds its thread about as long as
+    // the batch runs, and a wait behind it costs some 450 cycles before the next batch starts, in
+    // which a single issuer leaves the tensor pipe idle (5,200 cycles a step for 3,400 of MMAs);
+    // here the other batches run meanwhile.
+    if (lane == 0) {
+      auto wait = [&](uint32_t bar, uint32_t parity) {
+        if (!aborted && !mbar_wait(bar, parity, abort_flag)) aborted = true;
+      };
+      int r = 0, sidx = 0, qb = 0;   // the step's SNP tile, sample tile, Q buffer
+      uint32_t qpar = 0u;            // parity of the Q buffer's fill for that sample tile
+      for (int st = 0; st < nsteps; ++st) {
+        if (warp == H_WARP) {
+          if (st > 0) wait(HFREE, (uint32_t)(st - 1) & 1u);
+          if (r == 0) {
+            wait(QFULL(qb), qpar);
+            fence_async_smem();
+          }
         } else {
-          issue_abt(r, qb, st & 1, sidx > 0);
-          if (more) issue_h(r1, qb1, 1);
-          mma_commit(HFULL(1));
+          wait(ABREADY(st), (uint32_t)(st >> 1) & 1u);
+        }
+        if (aborted) break;
+        fence_after();
+        if (warp == H_WARP) {
+          issue_h(r, qb);
+          mma_commit(HFULL);
+        } else if (warp == AB_WARP) {
+          issue_ab(r, qb, st & 1, sidx);
+          mma_commit(ABFREE(st));
+          if (r + 1 == r_eff) mma_commit(QFREE(qb));   // the tile's last batch; its H's were done before
+        } else {
+          issue_t(r, st & 1, sidx);
+          mma_commit(ABFREE(st));
+        }
+        if (++r == r_eff) {
+          r = 0;
+          ++sidx;
+          if (++qb == NQ) { qb = 0; qpar ^= 1u; }
         }
       }
-      __syncwarp();
-      r = r1; sidx = sidx1; qb = qb1; qpar = qpar1;
     }
+    __syncwarp();
   } else {
     // ---------------------------------------------------------------- consumers
     const int hw = warp / (4 * HALF_WGS);       // half of every step
@@ -518,31 +537,32 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
     // the byte offset in the word and the field's position (at most 24 + 6 bits)
     const uint32_t goff = AL ? 0u : row_offset(a, jl >> 2);
     const uint32_t sh = 2u * (uint32_t)(jl & 3) + 8u * (goff & 3u);
-    int r = 0, sidx = 0, gstage = 0;
-    uint32_t hph = 0u, gph = 0u;
+    int r = 0, sidx = 0, gstage = 0, rprev = 0, sprev = 0;
+    uint32_t gph = 0u;
     for (int st = 0; st < nsteps; ++st) {
-      if (!mbar_wait(HFULL(hw), hph, abort_flag)) { aborted = true; break; }
-      hph ^= 1u;
-      if (!mbar_wait(GFULL(gstage), gph, abort_flag)) { aborted = true; break; }
+      if (!warp_wait(HFULL, (uint32_t)st & 1u, abort_flag)) { aborted = true; break; }
+      if (!warp_wait(GFULL(gstage), gph, abort_flag)) { aborted = true; break; }
       fence_after();
-      // T of the previous sample tile: its last T MMAs were committed before this H
-      if (hw == 1 && sub == 0 && r == 0 && sidx > 0) write_t(s_first + (int64_t)(sidx - 1) * a.n_split);
-
       const int64_t jglob = jb + (int64_t)r * TILE + jl;
       const uint8_t* gs = sm + OFF_G + gstage * G_TILE_BYTES + (jl >> 2) * G_ROW + colb + (goff & ~3u);
       uint8_t* ta = sm + OFF_A + (st & 1) * AB_TILE_BYTES;
       uint8_t* tb = sm + OFF_B + (st & 1) * AB_TILE_BYTES;
-      uint32_t hv[2][16], cv[2][16];
-      tmem_ld16(trow, hv[0]);
-      tmem_ld16(trow + HALF, cv[0]);
-      tmem_wait_ld();
+      // all of the warpgroup's H and Hc, then the buffer is free for the next step's
+      constexpr int NCH = WG_COLS / 16;
+      static_assert(NCH == 2, "the whole block of columns is held in registers");
+      uint32_t hv[NCH][16], cv[NCH][16];
 #pragma unroll
-      for (int c = 0; c < WG_COLS / 16; ++c) {
-        const int cur = c & 1;
-        if (c + 1 < WG_COLS / 16) {
-          tmem_ld16(trow + 16 * (c + 1), hv[cur ^ 1]);
-          tmem_ld16(trow + HALF + 16 * (c + 1), cv[cur ^ 1]);
-        }
+      for (int c = 0; c < NCH; ++c) {
+        tmem_ld16(trow + 16 * c, hv[c]);
+        tmem_ld16(trow + HALF + 16 * c, cv[c]);
+      }
+      tmem_wait_ld();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(HFREE);
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) {
+        const int cur = c;
         const int col0 = colb + 16 * c;
         uint32_t words[5];
         if constexpr (AL) {
@@ -580,38 +600,56 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
             bp[e >> 1] = F::mul(prmt(F::GB_LO, F::GB_HI, sel), xpair);
           }
         }
+        if (c == 0 && st > 1) {
+          // the a/b buffer's last batch, of step st - 2, is done
+          if (!warp_wait(ABFREE(st), (uint32_t)((st >> 1) - 1) & 1u, abort_flag)) { aborted = true; break; }
+          // ... and with it T of a sample tile that ended there (T alternates between two
+          // buffers: the current tile's is the other one or, with one SNP tile per CTA, the same
+          // one, whose next batch waits for this warpgroup's arrival below)
+          if (hw == 1 && sub == 0 && rprev == 0 && sprev > 0) {
+            fence_after();
+            write_t(sprev - 1);
+            fence_before();
+          }
+        }
         *reinterpret_cast<uint4*>(ta + off_ab(jl, col0)) = make_uint4(ap[0], ap[1], ap[2], ap[3]);
         *reinterpret_cast<uint4*>(ta + off_ab(jl, col0 + 8)) = make_uint4(ap[4], ap[5], ap[6], ap[7]);
         *reinterpret_cast<uint4*>(tb + off_ab(jl, col0)) = make_uint4(bp[0], bp[1], bp[2], bp[3]);
         *reinterpret_cast<uint4*>(tb + off_ab(jl, col0 + 8)) = make_uint4(bp[4], bp[5], bp[6], bp[7]);
-        if (c + 1 < WG_COLS / 16) tmem_wait_ld();
       }
+      if (aborted) break;
+      rprev = r;
+      sprev = sidx;
       fence_async_smem();
-      fence_before();
-      mbar_arrive(ABREADY(hw));
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(ABREADY(st));
+        mbar_arrive(GFREE(gstage));
+      }
       if (++r == r_eff) { r = 0; ++sidx; }
       if (++gstage == NG) { gstage = 0; gph ^= 1u; }
     }
   }
 
-  // ---- epilogue: wait for the last MMAs (the last step's commit is completion nsteps of
-  // hfull[1]; the prologue's was completion 0)
-  if (!aborted) {
-    if (!mbar_wait(HFULL(1), (uint32_t)(nsteps & 1), abort_flag)) aborted = true;
+  // ---- epilogue: wait for the last MMAs (the last step's commit covers everything)
+  if (!aborted && warp != LOAD_WARP) {
+    if (!mbar_wait(ABFREE(nsteps - 1), (uint32_t)((nsteps - 1) >> 1) & 1u, abort_flag)) aborted = true;
   }
   if (__syncthreads_or(aborted)) {
     if (tid == 0) atomicExch(a.err, ADX_ERR_TIMEOUT);
-    if (warp == PRODUCER_WARP) {
-      // MMAs may still be in flight: one more commit and bounded waits before freeing TMEM
+    if (warp >= H_WARP) {
+      // MMAs may still be in flight: one more commit and a bounded wait before TMEM is freed
       volatile int never = 0;
-      if (lane == 0) mma_commit(HFULL(0));
-      (void)mbar_wait(HFULL(0), 0u, &never);
-      (void)mbar_wait(HFULL(0), 1u, &never);
+      if (lane == 0) mma_commit(DRAIN(warp));
+      (void)mbar_wait(DRAIN(warp), 0u, &never);
     }
   } else {
     fence_after();
-    if (warp >= 4 && warp < 8 && HALF_WGS == 1) write_t(s_first + (int64_t)(n_my - 1) * a.n_split);
-    if (warp >= 8 && warp < 12 && HALF_WGS == 2) write_t(s_first + (int64_t)(n_my - 1) * a.n_split);
+    // the last tiles' T: the last one's, and with one SNP tile per CTA the one before it
+    if (warp >= 4 * HALF_WGS && warp < 4 * HALF_WGS + 4) {
+      if (r_eff == 1 && n_my > 1) write_t(n_my - 2);
+      write_t(n_my - 1);
+    }
     if (warp < 8) {
       // A/B of every SNP tile: warps 0-3 read A, warps 4-7 read B
       const int wg = warp >> 2, wq = warp & 3;
@@ -632,7 +670,7 @@ __global__ void __launch_bounds__(TPB, 1) em_sweep_tc_kernel(Args a) {
   fence_before();
   __syncthreads();
   fence_after();
-  if (warp == PRODUCER_WARP) {
+  if (warp == H_WARP) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
   }
 }

@@ -7,7 +7,7 @@
 namespace adx {
 namespace tc {
 
-constexpr uint32_t WAIT_LIMIT = 1u << 26;  // ~seconds of polling before giving up
+constexpr uint32_t WAIT_LIMIT = 1u << 24;  // polls before giving up: from a fraction of a second on
 
 // Shared-memory matrix descriptor, no swizzle, Blackwell version bit.
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
@@ -42,8 +42,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
                                           uint32_t limit = WAIT_LIMIT) {
   for (uint32_t it = 0; it < limit; ++it) {
     if (mbar_try(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (it > 64) __nanosleep(32);
+    if ((it & 15u) == 15u && *abort_flag) return false;
   }
   *abort_flag = 1;
   return false;

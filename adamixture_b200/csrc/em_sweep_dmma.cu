@@ -129,7 +129,7 @@ __device__ __forceinline__ double weight_b(uint32_t code) {
 }
 
 // fmin(fmax(x, lo), 1 - lo), lo > 0, by the bit patterns, which order as the values do: the
-// MMAs and the float64 comparisons share a pipe, and it is what bounds the sweep (29.1 -> 27.9
+// MMAs and the float64 comparisons share a pipe, and it is what bounds the sweep (29.1 -> 27.6
 // ms at N=100,000 x M=50,000, K=10). x comes out of an MMA: a NaN is the positive one and
 // goes to the upper bound where fmax would take it to the lower; the model is lost either way.
 __device__ __forceinline__ double clamp_bits(double x, double lo) {
@@ -151,26 +151,67 @@ __device__ __forceinline__ bool inside(const double (&x)[N], double lo) {
   return in;
 }
 
-// The genotype bytes of SNP rows g and g+8 of the chunk at jc for the thread's 8 samples
-// from s0 (0xFF, all missing, past N); rows past the matrix read its last row (those SNPs
-// are masked as missing by the caller).
-__device__ __forceinline__ void load_words(const uint8_t* __restrict__ G, int64_t N, int64_t rows, int64_t jc,
-                                           int g, int64_t s0, bool full8, uint64_t (&w)[2]) {
+// The genotype bytes of SNP rows g and g+8 of the chunk at jc for the thread's 8 samples from
+// s0. Rows past the matrix read its last row (those SNPs are masked as missing by the caller).
+// fetch: the aligned words that hold them, a chunk ahead of their use -- one 8-byte load where
+// every packed row is 8-byte aligned (VEC), else three words (byte loads through one thread
+// took the sweep from 27.9 to 37.2 ms at N=100,003 x M=50,000, K=10, and the log-likelihood from
+// 6.8 to 9.8 ms at N=50,003 x M=100,000, K=8: 28.3 and 7.0 ms with the words). Bytes past the
+// matrix are 0xFF.
+struct RowWords {
+  uint32_t w0, w1, w2;
+};
+__device__ __forceinline__ int64_t packed_row(int64_t rows, int64_t jc, int g, int h) {
+  return min((jc + g + 8 * h) >> 2, rows - 1);
+}
+template <bool VEC>
+__device__ __forceinline__ void fetch_rows(const uint8_t* __restrict__ G, int64_t N, int64_t rows, int64_t jc, int g,
+                                           int64_t s0, RowWords (&w)[2]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    const int64_t row = min(((jc + g + 8 * h) >> 2), rows - 1);
-    const uint8_t* src = G + row * N + s0;
-    if (full8) {
-      w[h] = __ldg(reinterpret_cast<const unsigned long long*>(src));
+    const int64_t at = packed_row(rows, jc, g, h) * N + s0, total = rows * N;
+    const uint8_t* p = G + at;
+    if (s0 >= N) {
+      w[h] = RowWords{~0u, ~0u, ~0u};
+    } else if (VEC) {   // s0 and N are multiples of 8
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+      w[h].w0 = v.x;
+      w[h].w1 = v.y;
     } else {
-      uint64_t v = 0;
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const uint64_t by = (s0 + u < N) ? (uint64_t)__ldg(src + u) : 0xFFull;
-        v |= by << (8 * u);
+      const uint8_t* q = p - (reinterpret_cast<uintptr_t>(p) & 3);
+      if (q >= G && at + 12 <= total) {
+        w[h].w0 = __ldg(reinterpret_cast<const uint32_t*>(q));
+        w[h].w1 = __ldg(reinterpret_cast<const uint32_t*>(q + 4));
+        w[h].w2 = __ldg(reinterpret_cast<const uint32_t*>(q + 8));
+      } else {
+        uint32_t v[3];
+        for (int c = 0; c < 3; ++c) {
+          v[c] = 0;
+          for (int b = 0; b < 4; ++b) {
+            const uint8_t* r = q + 4 * c + b;
+            v[c] |= (r >= G && r < G + total ? (uint32_t)__ldg(r) : 0xFFu) << (8 * b);
+          }
+        }
+        w[h] = RowWords{v[0], v[1], v[2]};
       }
-      w[h] = v;
     }
+  }
+}
+// join: the 8 bytes; samples past N are 0xFF (missing).
+template <bool VEC>
+__device__ __forceinline__ void join_rows(const uint8_t* __restrict__ G, int64_t N, int64_t rows, int64_t jc, int g,
+                                          int64_t s0, const RowWords (&w)[2], uint64_t (&out)[2]) {
+  if constexpr (VEC) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) out[h] = (uint64_t)w[h].w0 | ((uint64_t)w[h].w1 << 32);
+    return;
+  }
+  const uint64_t past = s0 + 8 <= N ? 0ull : s0 >= N ? ~0ull : ~0ull << (8 * (uint32_t)(N - s0));
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t at = (uint32_t)reinterpret_cast<uintptr_t>(G) + (uint32_t)packed_row(rows, jc, g, h) * (uint32_t)N + (uint32_t)s0;
+    const uint32_t sh = 8u * (at & 3u);
+    out[h] = ((uint64_t)__funnelshift_r(w[h].w0, w[h].w1, sh) | ((uint64_t)__funnelshift_r(w[h].w1, w[h].w2, sh) << 32)) | past;
   }
 }
 
@@ -255,7 +296,7 @@ struct Probs {
 // block in groups of 8 chunks of 16 SNPs, then the sub-tile's T partials.
 // LL: also multiply every entry's log-likelihood factor into (prod, ex), in the order and
 // arithmetic of loglik_dmma_kernel, so the CTA's partial equals that kernel's.
-template <int KS, bool LL, int TL>
+template <int KS, bool LL, int TL, bool VEC>
 __device__ __forceinline__ void sweep_subtile(const Args& a, const Prob& pr, int64_t st, int split, int mblk,
                                               int& chunk_no, double* sm, double& prod, int& ex) {
   using L = Lay<TL>;
@@ -298,9 +339,8 @@ __device__ __forceinline__ void sweep_subtile(const Args& a, const Prob& pr, int
     // this thread's 8 consecutive samples; the first chunk's genotype words are loaded
     // here and each chunk loads the next one's, a chunk ahead of their use
     const int64_t s0 = i0 + warp * WS + 8 * t;
-    const bool full8 = pr.vec && (s0 + 8 <= N);
-    uint64_t wnext[2];
-    load_words(pr.G, N, rows, j0, g, s0, full8, wnext);
+    RowWords wnext[2];
+    fetch_rows<VEC>(pr.G, N, rows, j0, g, s0, wnext);
 
     for (int64_t gj = j0; gj < j1; gj += GS) {
       const int gn = (int)min((int64_t)GS, j1 - gj);
@@ -313,8 +353,9 @@ __device__ __forceinline__ void sweep_subtile(const Args& a, const Prob& pr, int
       for (int ch = 0; ch < nch; ++ch) {
         const int64_t jc = gj + ch * CH;
         const double* pc = pt + ch * CH * PSTR;
-        uint64_t w[2] = {wnext[0], wnext[1]};
-        if (jc + CH < j1) load_words(pr.G, N, rows, jc + CH, g, s0, full8, wnext);
+        uint64_t w[2];
+        join_rows<VEC>(pr.G, N, rows, jc, g, s0, wnext, w);
+        if (jc + CH < j1) fetch_rows<VEC>(pr.G, N, rows, jc + CH, g, s0, wnext);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           // SNPs past the block end are missing (code 3)
@@ -520,7 +561,7 @@ __device__ __forceinline__ void sweep_subtile(const Args& a, const Prob& pr, int
 // LL (single problem only): the sweep also sums the log-likelihood of its input (P, Q) into
 // a.llp[blockIdx.x], bit-identical to loglik_dmma_kernel's partials.
 // TL: the shared-memory layout (Lay<TL>); it sets how many CTAs share an SM.
-template <int KS, int MAXP, bool LL, int TL>
+template <int KS, int MAXP, bool LL, int TL, bool VEC>
 __global__ void __launch_bounds__(TPB, Lay<TL>::OCC) em_sweep_dmma_kernel(Args a, Probs<MAXP> ps) {
   static_assert(!LL || MAXP == 1, "the log-likelihood rides on single-problem sweeps");
   extern __shared__ __align__(16) double sm[];
@@ -533,17 +574,17 @@ __global__ void __launch_bounds__(TPB, Lay<TL>::OCC) em_sweep_dmma_kernel(Args a
     const Prob pr = ps.p[pi];
     for (int64_t st = split; st < a.n_stile; st += a.n_split) {
       if constexpr (MAXP == 1) {
-        sweep_subtile<KS, LL, TL>(a, pr, st, split, mblk, chunk_no, sm, prod, ex);
+        sweep_subtile<KS, LL, TL, VEC>(a, pr, st, split, mblk, chunk_no, sm, prod, ex);
       } else if constexpr (Lay<TL>::KSMAX <= 2) {
         // the host launches this layout only for batches whose every K is <= 8
-        if (((pr.K + 3) >> 2) == 1) sweep_subtile<1, false, TL>(a, pr, st, split, mblk, chunk_no, sm, prod, ex);
-        else sweep_subtile<2, false, TL>(a, pr, st, split, mblk, chunk_no, sm, prod, ex);
+        if (((pr.K + 3) >> 2) == 1) sweep_subtile<1, false, TL, VEC>(a, pr, st, split, mblk, chunk_no, sm, prod, ex);
+        else sweep_subtile<2, false, TL, VEC>(a, pr, st, split, mblk, chunk_no, sm, prod, ex);
       } else {
         switch ((pr.K + 3) >> 2) {
-          case 1: sweep_subtile<1, false, TL>(a, pr, st, split, mblk, chunk_no, sm, prod, ex); break;
-          case 2: sweep_subtile<2, false, TL>(a, pr, st, split, mblk, chunk_no, sm, prod, ex); break;
-          case 3: sweep_subtile<3, false, TL>(a, pr, st, split, mblk, chunk_no, sm, prod, ex); break;
-          default: sweep_subtile<4, false, TL>(a, pr, st, split, mblk, chunk_no, sm, prod, ex); break;
+          case 1: sweep_subtile<1, false, TL, VEC>(a, pr, st, split, mblk, chunk_no, sm, prod, ex); break;
+          case 2: sweep_subtile<2, false, TL, VEC>(a, pr, st, split, mblk, chunk_no, sm, prod, ex); break;
+          case 3: sweep_subtile<3, false, TL, VEC>(a, pr, st, split, mblk, chunk_no, sm, prod, ex); break;
+          default: sweep_subtile<4, false, TL, VEC>(a, pr, st, split, mblk, chunk_no, sm, prod, ex); break;
         }
       }
     }
@@ -565,10 +606,10 @@ __global__ void __launch_bounds__(TPB, Lay<TL>::OCC) em_sweep_dmma_kernel(Args a
 constexpr int LL_SMEM_DOUBLES = P_OFF + GS * PSTR + WARPS;
 constexpr size_t LL_SMEM_BYTES = sizeof(double) * LL_SMEM_DOUBLES;
 
-template <int KS>
+template <int KS, bool VEC>
 __global__ void __launch_bounds__(TPB, 2) loglik_dmma_kernel(Args a, const uint8_t* __restrict__ G,
                                                              const double* __restrict__ P,
-                                                             const double* __restrict__ Q, int K, int vec,
+                                                             const double* __restrict__ Q, int K,
                                                              double* __restrict__ partial) {
   extern __shared__ __align__(16) double sm[];
   double* qt = sm + Q_OFF;
@@ -593,9 +634,8 @@ __global__ void __launch_bounds__(TPB, 2) loglik_dmma_kernel(Args a, const uint8
       qt[r * QSTR + (k ^ qsw(r))] = (i < N && k < K) ? Q[i * K + k] : 0.0;
     }
     const int64_t s0 = i0 + warp * WS + 8 * t;
-    const bool full8 = vec && (s0 + 8 <= N);
-    uint64_t wnext[2];
-    load_words(G, N, rows, j0, g, s0, full8, wnext);
+    RowWords wnext[2];
+    fetch_rows<VEC>(G, N, rows, j0, g, s0, wnext);
     for (int64_t gj = j0; gj < j1; gj += GS) {
       const int gn = (int)min((int64_t)GS, j1 - gj);
       __syncthreads();
@@ -608,8 +648,9 @@ __global__ void __launch_bounds__(TPB, 2) loglik_dmma_kernel(Args a, const uint8
       for (int ch = 0; ch < nch; ++ch) {
         const int64_t jc = gj + ch * CH;
         const double* pc = pt + ch * CH * PSTR;
-        uint64_t w[2] = {wnext[0], wnext[1]};
-        if (jc + CH < j1) load_words(G, N, rows, jc + CH, g, s0, full8, wnext);
+        uint64_t w[2];
+        join_rows<VEC>(G, N, rows, jc, g, s0, wnext, w);
+        if (jc + CH < j1) fetch_rows<VEC>(G, N, rows, jc + CH, g, s0, wnext);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (jc + g + 8 * h >= j1) w[h] |= 0x0303030303030303ull << (2 * (g & 3));
@@ -635,7 +676,7 @@ __global__ void __launch_bounds__(TPB, 2) loglik_dmma_kernel(Args a, const uint8
             mma_f64(hacc[nt], ph[KS - 1][0], ph[KS - 1][1], qt[qrow * QSTR + ((4 * (KS - 1) + t) ^ qsw(qrow))]);
         }
         // one vote for the chunk's 16 values a thread: the clamps are rarely needed. They and a
-        // renormalisation per 4 factors instead of 8 took 8.08 ms where this takes 6.8 (N=50,000 x
+        // renormalisation per 4 factors instead of 8 took 8.08 ms where this takes 6.5 (N=50,000 x
         // M=100,000, K=8); a vote per tile of 4 was slower than the clamps (8.8 ms)
         if (__all_sync(0xffffffffu, inside(hacc[0], LL_CLAMP) && inside(hacc[1], LL_CLAMP) &&
                                         inside(hacc[2], LL_CLAMP) && inside(hacc[3], LL_CLAMP))) {
@@ -656,23 +697,30 @@ __global__ void __launch_bounds__(TPB, 2) loglik_dmma_kernel(Args a, const uint8
 int dmma_plan_width() { return dm::W; }
 int dmma_plan_chunk() { return dm::CH; }
 
-template <int KS, int MAXP, bool LL, int TL>
-static int dmma_launch(const dm::Args& a, const dm::Probs<MAXP>& ps, cudaStream_t st) {
+template <int KS, int MAXP, bool LL, int TL, bool VEC>
+static int dmma_launch_as(const dm::Args& a, const dm::Probs<MAXP>& ps, cudaStream_t st) {
   static bool attr_set[64] = {false};
   int dev = 0;
   ADX_CUDA_TRY(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    ADX_CUDA_TRY(cudaFuncSetAttribute(dm::em_sweep_dmma_kernel<KS, MAXP, LL, TL>,
+    ADX_CUDA_TRY(cudaFuncSetAttribute(dm::em_sweep_dmma_kernel<KS, MAXP, LL, TL, VEC>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dm::Off<TL>::BYTES));
     // all of the unified L1/shared storage as shared memory, so that OCC CTAs fit on an SM
-    ADX_CUDA_TRY(cudaFuncSetAttribute(dm::em_sweep_dmma_kernel<KS, MAXP, LL, TL>,
+    ADX_CUDA_TRY(cudaFuncSetAttribute(dm::em_sweep_dmma_kernel<KS, MAXP, LL, TL, VEC>,
                                       cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set[dev] = true;
   }
-  dm::em_sweep_dmma_kernel<KS, MAXP, LL, TL>
+  dm::em_sweep_dmma_kernel<KS, MAXP, LL, TL, VEC>
       <<<(unsigned)(a.n_split * a.nmb), dm::TPB, dm::Off<TL>::BYTES, st>>>(a, ps);
   ADX_LAUNCH_CHECK();
   return ADX_OK;
+}
+
+template <int KS, int MAXP, bool LL, int TL>
+static int dmma_launch(const dm::Args& a, const dm::Probs<MAXP>& ps, cudaStream_t st) {
+  bool vec = true;
+  for (int p = 0; p < ps.n; ++p) vec = vec && ps.p[p].vec;
+  return vec ? dmma_launch_as<KS, MAXP, LL, TL, true>(a, ps, st) : dmma_launch_as<KS, MAXP, LL, TL, false>(a, ps, st);
 }
 
 // The layout each (device, K) launches its float64 sweeps with, set by adx_dmma_tile_set
@@ -772,25 +820,27 @@ int dmma_loglik(const uint8_t* G, const double* P, const double* Q, int64_t M, i
   if (!partial) return ADX_OK;
   const dm::Args a{M, N, n_stile, n_split, n_mblk, mb, nullptr};
   const int vec = dmma_vec(G, N);
-#define ADX_LL_DM(KS)                                                                                          \
+#define ADX_LL_AS(KS, VEC)                                                                                      \
   {                                                                                                            \
     static bool attr_set[64] = {false};                                                                        \
     int dev = 0;                                                                                               \
     ADX_CUDA_TRY(cudaGetDevice(&dev));                                                                         \
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {                                                              \
-      ADX_CUDA_TRY(cudaFuncSetAttribute(dm::loglik_dmma_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                        (int)dm::LL_SMEM_BYTES));                                              \
+      ADX_CUDA_TRY(cudaFuncSetAttribute(dm::loglik_dmma_kernel<KS, VEC>,                                       \
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dm::LL_SMEM_BYTES)); \
       attr_set[dev] = true;                                                                                    \
     }                                                                                                          \
-    dm::loglik_dmma_kernel<KS><<<(unsigned)(n_split * n_mblk), dm::TPB, dm::LL_SMEM_BYTES, st>>>(a, G, P, Q, K,  \
-                                                                                              vec, partial);   \
+    dm::loglik_dmma_kernel<KS, VEC><<<(unsigned)(n_split * n_mblk), dm::TPB, dm::LL_SMEM_BYTES, st>>>(          \
+        a, G, P, Q, K, partial);                                                                               \
   }
+#define ADX_LL_DM(KS) { if (vec) ADX_LL_AS(KS, true) else ADX_LL_AS(KS, false) }
   switch ((K + 3) / 4) {
     case 1: ADX_LL_DM(1) break;
     case 2: ADX_LL_DM(2) break;
     case 3: ADX_LL_DM(3) break;
     default: ADX_LL_DM(4) break;
   }
+#undef ADX_LL_AS
 #undef ADX_LL_DM
   ADX_LAUNCH_CHECK();
   return ADX_OK;

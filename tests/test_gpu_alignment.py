@@ -140,3 +140,27 @@ def test_float32_loglik_of_small_k(ops, K):
         assert abs(float(ref) - L) <= tol
         for off in (1, 6, 15):
             assert torch.equal(ops.loglik_device(placed(packed, off), P32, Q32, M, "f32"), ref), off
+
+
+@pytest.mark.parametrize("K", [1, 4, 7, 8, 10, 16])
+def test_float64_sweep_and_loglik_do_not_depend_on_alignment(ops, K):
+    # the aligned kernels (N % 8 = 0 at offset 0) against the word loads at every other address,
+    # and ragged cohorts at all of them; the folded check too
+    for N, M in ((256, 40), (264, 130), (105, 70), (515, 517)):
+        G, P, Q = cohort(N, M, K, K + N + M)
+        packed = orc.pack(G)
+        Pd, Qd = torch.from_numpy(P).cuda(), torch.from_numpy(Q).cuda()
+        ref = ll = None
+        for off in (0, 1, 6, 8, 13):
+            X = placed(packed, off)
+            got = ops.em_stats(X, Pd, Qd, M, "f64")
+            L = ops.loglik_device(X, Pd, Qd, M, "f64")
+            ws = ops.em_workspace(M, N, K, "f64", X.device)
+            ops.em_sweep_loglik(X, Pd, Qd, M, ws)
+            assert torch.equal(ops.em_loglik_from_sweep(ws, M, N, K), L)
+            if ref is None:
+                ref, ll = got, L
+                want = orc.em_stats(G, P, Q)[:3]
+                assert all(np.abs(g.cpu().numpy() - w).max() <= 1e-11 * np.abs(w).max() for g, w in zip(got, want))
+                assert abs(float(L) - orc.loglik(G, P, Q)) <= 1e-12 * abs(float(L))
+            assert all(torch.equal(g, r) for g, r in zip(got, ref)) and torch.equal(L, ll), off

@@ -801,10 +801,13 @@ static int launch_update_from(const EmPlan& pl, const R* ABp, const R* Tp, int m
   const int threads = 128;
   // A warp per row where one thread's walk over the partials would be the launch's time: few
   // rows, many partials. One thread per sample took 130 us of a 150 us iteration at N=105 x
-  // M=8,451, K=7 (529 partials), and 2.70 -> 2.64 ms at N=10,007 (224 partials); at N=20,000 (136
-  // partials) the threads' neighbouring rows make up for it: 3.97 against 4.02 ms.
-  const int gp = pl.M < 16384 && pl.n_split >= 32 ? 32 : 1;
-  const int gq = pl.N < 16384 && pl.n_mblk >= 32 ? 32 : 1;
+  // M=8,451, K=7 (529 partials), and 2.70 -> 2.64 ms at N=10,007 (224 partials); with fewer
+  // partials or more rows the threads' neighbouring rows make up for it: at N=15,912 x M=9,908,
+  // K=16 (45 and 38 partials) 1.18 ms against 1.21, at N=20,000 (136) 3.97 against 4.02.
+  auto lanes = [](int64_t rows, int parts) {
+    return (rows <= 4096 && parts >= 32) || (rows < 16384 && parts >= 128) ? 32 : 1;
+  };
+  const int gp = lanes(pl.M, pl.n_split), gq = lanes(pl.N, pl.n_mblk);
   const unsigned p_blocks = (unsigned)ceil_div(pl.M * gp, threads);
   const dim3 grid(p_blocks + (unsigned)ceil_div(pl.N * gq, threads));
 #define LAUNCH(KM)                                                                          \

@@ -95,6 +95,7 @@ struct Args {
   long long* sc;           // [rows][L] code sums (rows: S1 - 3 S2)
   long long* sm;           // [rows][L] flag sums
   int* err;
+  uint32_t polls;          // limit of a wait
 };
 
 __host__ __device__ inline int digit_bytes(int Lb) { return BLK * NDIG * Lb; }
@@ -142,25 +143,38 @@ __device__ __forceinline__ void arrive_expect(uint32_t bar, uint32_t bytes) {
                : "memory");
 }
 
-// Bounded wait of a whole warp. It never blocks once the CTA has given up (a timeout raises
-// the abort word): every warp then runs its loop to the end without waiting, so that each
-// named barrier still gets all its arrivals, and the result is discarded.
-__device__ __forceinline__ void warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  for (uint32_t it = 0; it < POLLS; ++it) {
-    if (tc::mbar_try(bar, parity)) return;
-    if ((it & 15u) == 15u && *abort_flag) return;
+// Bounded wait of a whole warp. False once it has run out of polls, which raises the abort word,
+// or another warp has given up.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t polls) {
+  for (uint32_t it = 0; it < polls; ++it) {
+    if (tc::mbar_try(bar, parity)) return true;
+    if ((it & 15u) == 0u && *abort_flag) return false;
   }
   *abort_flag = 1;
+  return false;
 }
 
-// A stage's hand-over from the unpack group to the MMA warp: a named barrier (a hardware
-// barrier wakes the waiter in tens of cycles; an mbarrier here cost several hundred per stage).
+// A stage's hand-over from the unpack group to the MMA warp: a named barrier, a generation per
+// fill of the stage (1.95 ms a product at N = M = 100,000, L=20; an mbarrier here takes 2.25 to
+// 2.35, whichever way its waiter polls). A named barrier has no limit of its own and counts
+// arrivals without asking whose they are, so every generation must get exactly one arrival of each
+// of its 9 warps and none before the previous generation of that stage is complete:
+// - unpack and MMA warps never leave their loops early: after a wait that has run out they go on to
+//   the end, where the results are discarded;
+// - an unpack warp comes to a stage's next generation only when the MMA warp has passed the
+//   one before: the AEMPTY wait proves it, and where that has been given up, `joined` (the
+//   stages the MMA warp has passed) is waited for instead. That always ends: the warps whose
+//   arrivals the MMA warp lacks are at its stage or before it, so what they wait for it has
+//   already written.
 constexpr int HANDOVER = 32 * (GROUP_WARPS + 1);
 __device__ __forceinline__ void stage_arrive(int st) {
   asm volatile("bar.arrive %0, %1;" ::"r"(1 + st), "n"(HANDOVER) : "memory");
 }
 __device__ __forceinline__ void stage_sync(int st) {
   asm volatile("bar.sync %0, %1;" ::"r"(1 + st), "n"(HANDOVER) : "memory");
+}
+__device__ __forceinline__ void wait_joined(const volatile int* joined, int stages) {
+  for (uint32_t it = 0; it < POLLS && *joined < stages; ++it) __nanosleep(200);
 }
 
 // 64 packed rows from row0 x 256 samples from i0 into a slot, by the load warp. AL: every
@@ -236,6 +250,7 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
   const uint32_t DONE = bars + 8u * (uint32_t)(N_BARS - 1);
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(ctl + 8 * N_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(ctl + 8 * N_BARS + 4);
+  volatile int* joined = reinterpret_cast<volatile int*>(ctl + 8 * N_BARS + 8);   // stages the MMA warp has passed
 
   int64_t b = blockIdx.x;
   const int64_t tile = b % a.tiles; b /= a.tiles;
@@ -251,6 +266,7 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
   }
   if (tid == 0) {
     *abort_flag = 0;
+    *joined = 0;
     for (int s = 0; s < NSLOT; ++s) {
       // 32 asynchronous and 32 plain arrivals of the load warp, and the bulk copies' expect
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 65;" ::"r"(FULL(s)));
@@ -266,11 +282,12 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
   const uint32_t tmem = *tmem_holder;
   const uint32_t col_a = tmem + 4u * (uint32_t)n4;      // A stages: per stage and tile 16 code, 16 flag columns
 
+  int loaded = 0;   // blocks that the load warp has asked for
   if (warp == LOAD_WARP) {
     int slot = 0;
     uint32_t fill = 0;   // how often the ring has wrapped
     for (int q = 0; q < nq; ++q) {
-      if (fill > 0) warp_wait(EMPTY(slot), (fill - 1) & 1u, abort_flag);
+      if (fill > 0 && !warp_wait(EMPTY(slot), (fill - 1) & 1u, abort_flag, a.polls)) break;
       uint8_t* gs = sm + slot * slot_bytes;
       const int64_t blk = q0 + q;
       if (lane == 0) {
@@ -282,6 +299,7 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
       load_g<AL>(a, (ROWS ? tile * OWN : blk * BLK) >> 2, ROWS ? blk * BLK : tile * OWN, gs);
       cp_async_arrive(FULL(slot));
       mbar_arrive(FULL(slot));
+      ++loaded;
       if (++slot == NSLOT) { slot = 0; ++fill; }
     }
   } else if (warp == MMA_WARP) {
@@ -289,7 +307,7 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
     int slot = 0, st = 0;
     uint32_t fill = 0;
     for (int q = 0; q < nq; ++q) {
-      warp_wait(FULL(slot), fill & 1u, abort_flag);
+      warp_wait(FULL(slot), fill & 1u, abort_flag, a.polls);
       const uint32_t sb = smem_u32(sm + slot * slot_bytes + G_BYTES);
       const uint64_t dc = tc::sdesc(sb, 128, 256), dm = ROWS ? dc : tc::sdesc(sb + dbytes, 128, 256);
       const uint64_t step = (uint64_t)(32 * n4) >> 4;   // one 32-entry step of a digit tile
@@ -310,13 +328,14 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
           }
           mma_commit(AEMPTY(st));
           if (ks == KSTEPS - 1) mma_commit(EMPTY(slot));
+          *joined = q * KSTEPS + ks + 1;
         }
         __syncwarp();
         if (++st == a.nstage) st = 0;
       }
       if (++slot == NSLOT) { slot = 0; ++fill; }
     }
-    if (lane == 0) mma_commit(DONE);
+    if (lane == 0) mma_commit(DONE);   // also after a wait that ran out: covers the MMAs issued
     __syncwarp();
   } else {
     const int wq = warp & 3, t = (warp >> 2) & 1, grp = warp / GROUP_WARPS;
@@ -335,7 +354,7 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
     int slot = 0, st = 0, turn = 0;
     uint32_t fill = 0, sfill = 0;
     for (int q = 0; q < nq; ++q) {
-      warp_wait(FULL(slot), fill & 1u, abort_flag);
+      warp_wait(FULL(slot), fill & 1u, abort_flag, a.polls);
       const uint8_t* gs = sm + slot * slot_bytes;
       for (int ks = 0; ks < KSTEPS; ++ks) {
         const bool mine = turn == grp;
@@ -375,7 +394,10 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
           x[c] &= 0x03030303u;
           m[c] = x[c] & (x[c] >> 1) & 0x01010101u;
         }
-        if (my_fill > 0) warp_wait(AEMPTY(my_st), (my_fill - 1) & 1u, abort_flag);
+        if (my_fill > 0) {
+          if (!warp_wait(AEMPTY(my_st), (my_fill - 1) & 1u, abort_flag, a.polls))
+            wait_joined(joined, q * KSTEPS + ks - a.nstage + 1);
+        }
         fence_after();
         const uint32_t as = col_a + lanes + 64u * (uint32_t)my_st + 32u * (uint32_t)t;
         tmem_st16(as, x);
@@ -387,19 +409,20 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
       if (++slot == NSLOT) { slot = 0; ++fill; }
     }
   }
-  warp_wait(DONE, 0u, abort_flag);
+  warp_wait(DONE, 0u, abort_flag, a.polls);
   if (__syncthreads_or(*abort_flag)) {
-    // a bounded wait ran out: before the block ends, the copies and MMAs in flight land (these
-    // waits are bounded too)
+    // a wait ran out: before the block ends, the copies and MMAs in flight land (these waits are
+    // bounded too)
     if (tid == 0) atomicExch(a.err, ADX_ERR_TIMEOUT);
+    volatile int never = 0;
     if (warp == LOAD_WARP) {
       asm volatile("cp.async.wait_all;" ::: "memory");
-      volatile int never = 0;
       for (int s = 0; s < NSLOT; ++s) {
-        const int fills = (nq - s + NSLOT - 1) / NSLOT;
-        if (fills > 0) warp_wait(FULL(s), (uint32_t)(fills - 1) & 1u, &never);
+        const int fills = (loaded - s + NSLOT - 1) / NSLOT;
+        if (fills > 0) warp_wait(FULL(s), (uint32_t)(fills - 1) & 1u, &never, POLLS);
       }
-      warp_wait(DONE, 0u, &never);
+    } else if (warp == MMA_WARP) {
+      warp_wait(DONE, 0u, &never, POLLS);
     }
   } else {
     fence_after();
@@ -646,7 +669,7 @@ static_assert(NSLOT * (G_BYTES + 2 * BLK * NDIG * LB_MAX) + 8 * N_BARS + 16 + 12
 
 template <bool ROWS>
 static int product(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* F, int L, int accumulate,
-                   float* out, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+                   float* out, void* workspace, size_t workspace_bytes, cudaStream_t st, uint32_t polls = POLLS) {
   const int64_t n_rows = ROWS ? M : N, n_red = ROWS ? N : M;
   const Plan p = plan(n_rows, n_red, L, ROWS);
   if (!workspace || workspace_bytes < p.bytes) return ADX_ERR_WORKSPACE;
@@ -664,7 +687,7 @@ static int product(const uint8_t* G, int64_t M, int64_t N, const float* f, const
   ADX_LAUNCH_CHECK();
   digit_kernel<ROWS><<<(unsigned)(db < cap ? db : cap), 256, 0, st>>>(F, f, n_red, L, p.Lb, p.n_pass, p.n_blk, h, dc, dm);
   ADX_LAUNCH_CHECK();
-  const Args a{G, M, N, dc, dm, L, p.Lb, p.n_pass, p.n_blk, p.tiles, p.n_split, p.nstage, sc, sm, &h->err};
+  const Args a{G, M, N, dc, dm, L, p.Lb, p.n_pass, p.n_blk, p.tiles, p.n_split, p.nstage, sc, sm, &h->err, polls};
   const bool al = (N & 15) == 0 && (reinterpret_cast<uintptr_t>(G) & 15) == 0;
   const int rc = al ? launch<ROWS, true>(a, st) : launch<ROWS, false>(a, st);
   if (rc) return rc;
@@ -707,5 +730,19 @@ extern "C" int adx_rsvd_cols(const uint8_t* G, int64_t M, int64_t N, const float
   }
   const int rc = rt::product<false>(G, M, N, f, Y, L, accumulate, Z, workspace, workspace_bytes, as_stream(stream));
   if (rc == ADX_ERR_WORKSPACE) adx_set_message("adx_rsvd_cols: workspace too small");
+  return rc;
+}
+
+extern "C" int adx_rsvd_wait_selftest(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* F, int L,
+                                      int cols, uint32_t limit, float* out, void* workspace, size_t workspace_bytes,
+                                      void* stream) {
+  if (!G || !f || !F || !out || M <= 0 || N <= 0 || L < 1 || L > rt::L_MAX || limit > rt::POLLS) {
+    adx_set_message("adx_rsvd_wait_selftest: bad argument");
+    return ADX_ERR_ARG;
+  }
+  cudaStream_t st = as_stream(stream);
+  const int rc = cols ? rt::product<false>(G, M, N, f, F, L, 0, out, workspace, workspace_bytes, st, limit)
+                      : rt::product<true>(G, M, N, f, F, L, 0, out, workspace, workspace_bytes, st, limit);
+  if (rc == ADX_ERR_WORKSPACE) adx_set_message("adx_rsvd_wait_selftest: workspace too small");
   return rc;
 }

@@ -268,6 +268,11 @@ int adx_rsvd_rows_ws(const uint8_t* G, int64_t M, int64_t N, const float* f, con
 int adx_rsvd_cols(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* Y, int L,
                   int accumulate, float* Z, void* workspace, size_t workspace_bytes,
                   void* stream);
+/* Self-test of these products' bounded waits: one product (cols = 0: rows, else cols) whose
+ * waits each give up after `limit` polls (at most the products' own limit). Where one runs out
+ * the kernel ends by itself and every entry of `out` is NaN; limit = 0: every wait does. */
+int adx_rsvd_wait_selftest(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* F, int L, int cols,
+                           uint32_t limit, float* out, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Batched bounded least squares, float64, one warp per row: X[m] = argmin over
  * lower <= x <= upper of 1/2 x'Ax - B[m]'x by block principal pivoting, A [K][K] shared.

@@ -1,0 +1,61 @@
+"""GPU checks of the pipeline of the integer tensor-core products: shapes whose CTAs walk many
+blocks, so that the three load slots wrap and every A stage is filled several times at each
+stage count (2, 3 and 4, set by the factor's width), and what a product does when a wait runs
+out.
+
+Tolerance: as in test_gpu_rsvd_tc.py; the reference is float64."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops(cuda):
+    from adamixture_b200 import ops as _ops
+
+    return _ops
+
+
+def cohort(N, M, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    g = torch.randint(0, 4, ((M + 3) // 4 * 4, N), generator=gen, device="cuda", dtype=torch.uint8)
+    g[M:] = 0
+    q = g.view(-1, 4, N)
+    packed = (q[:, 0] | q[:, 1] << 2 | q[:, 2] << 4 | q[:, 3] << 6).contiguous()
+    f = torch.rand(M, generator=gen, device="cuda")
+    X = (g[:M].double() - 2.0 * f.double()[:, None]).masked_fill_(g[:M] == 3, 0.0)
+    return packed, f, X, gen
+
+
+# rows: a CTA per 256 SNPs walks every block of samples (9 and 4); cols: 4 to 9 of the SNPs'
+@pytest.mark.parametrize("N,M,L", [(2051, 38003, 16), (2048, 38000, 20), (2051, 38003, 24), (1003, 40011, 26)])
+def test_many_blocks_a_cta(ops, N, M, L):
+    G, f, X, gen = cohort(N, M, N + L)
+    B = torch.randn((N, L), generator=gen, device="cuda")
+    Y = torch.randn((M, L), generator=gen, device="cuda")
+    for got, ref, n, F, terms in ((ops.rsvd_rows(G, f, B, M), X @ B.double(), N, B, 2),
+                                  (ops.rsvd_cols(G, f, Y, M), X.T @ Y.double(), M, Y, 8)):
+        tol = terms * n * 2.0 ** -30 * F.abs().amax(0).double() + 2.0 ** -23 * ref.abs()
+        assert bool(((got.double() - ref).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("cols", [0, 1])
+def test_a_wait_that_runs_out(ops, cols):
+    # no wait gets a poll: every warp leaves its loop, the kernel ends by itself and says so in
+    # every entry; the next product is not affected
+    from adamixture_b200._lib import call, query_size
+
+    N, M, L = 1003, 40011, 20
+    G, f, X, gen = cohort(N, M, 3)
+    F = torch.randn((M if cols else N, L), generator=gen, device="cuda")
+    product = ops.rsvd_cols if cols else ops.rsvd_rows
+    before = product(G, f, F, M)
+    ws = torch.empty(query_size("adx_rsvd_workspace_bytes", M, N, L), dtype=torch.uint8, device="cuda")
+    out = torch.zeros_like(before)
+    call("adx_rsvd_wait_selftest", G.data_ptr(), M, N, f.data_ptr(), F.data_ptr(), L, cols, 0, out.data_ptr(),
+         ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    assert bool(torch.isnan(out).all())
+    assert torch.equal(product(G, f, F, M), before)
+    assert np.isfinite(before.cpu().numpy()).all()

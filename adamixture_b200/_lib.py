@@ -66,6 +66,7 @@ SIGNATURES: dict[str, list] = {
     "adx_rsvd_rows_ws": [P, I64, I64, P, P, c_int, P, P, c_size_t, P],
     "adx_rsvd_workspace_bytes": [I64, I64, c_int, P],
     "adx_rsvd_cols": [P, I64, I64, P, P, c_int, c_int, P, P, c_size_t, P],
+    "adx_rsvd_status": [P, c_size_t, P, P],
     "adx_rsvd_wait_selftest": [P, I64, I64, P, P, c_int, c_int, c_uint32, P, P, c_size_t, P],
     "adx_bvls": [P, P, I64, c_int, c_double, c_double, P, P],
     "adx_grad_hess_q": [P, I64, I64, c_int, P, P, P, P, P],

@@ -94,7 +94,8 @@ struct Args {
   int nstage;
   long long* sc;           // [rows][L] code sums (rows: S1 - 3 S2)
   long long* sm;           // [rows][L] flag sums
-  int* err;
+  int* err;                // status of this product
+  int* sticky;             // and of the workspace, until it is read
   uint32_t polls;          // limit of a wait
 };
 
@@ -413,7 +414,10 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
   if (__syncthreads_or(*abort_flag)) {
     // a wait ran out: before the block ends, the copies and MMAs in flight land (these waits are
     // bounded too)
-    if (tid == 0) atomicExch(a.err, ADX_ERR_TIMEOUT);
+    if (tid == 0) {
+      atomicExch(a.err, ADX_ERR_TIMEOUT);
+      atomicExch(a.sticky, ADX_ERR_TIMEOUT);
+    }
     volatile int never = 0;
     if (warp == LOAD_WARP) {
       asm volatile("cp.async.wait_all;" ::: "memory");
@@ -651,7 +655,7 @@ static Plan plan(int64_t n_rows, int64_t n_red, int L, bool rows) {
   p.head = pad(sizeof(Head));
   p.digits = pad((size_t)p.n_pass * p.n_blk * digit_bytes(p.Lb));
   p.sums = pad((size_t)n_rows * L * sizeof(long long));
-  p.bytes = p.head + (rows ? 1 : 2) * p.digits + 2 * p.sums + ALIGN;
+  p.bytes = ALIGN + p.head + (rows ? 1 : 2) * p.digits + 2 * p.sums + ALIGN;
   return p;
 }
 
@@ -667,13 +671,20 @@ static int launch(const Args& a, cudaStream_t st) {
 }
 static_assert(NSLOT * (G_BYTES + 2 * BLK * NDIG * LB_MAX) + 8 * N_BARS + 16 + 128 <= 227 * 1024, "shared memory");
 
+// The workspace's first aligned word is its status, which only adx_rsvd_status clears; the
+// parts of a product follow.
+static uint8_t* aligned(void* workspace) {
+  return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(workspace) + ALIGN - 1) & ~uintptr_t(ALIGN - 1));
+}
+
 template <bool ROWS>
 static int product(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* F, int L, int accumulate,
                    float* out, void* workspace, size_t workspace_bytes, cudaStream_t st, uint32_t polls = POLLS) {
   const int64_t n_rows = ROWS ? M : N, n_red = ROWS ? N : M;
   const Plan p = plan(n_rows, n_red, L, ROWS);
   if (!workspace || workspace_bytes < p.bytes) return ADX_ERR_WORKSPACE;
-  uint8_t* w = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(workspace) + ALIGN - 1) & ~uintptr_t(ALIGN - 1));
+  int* sticky = reinterpret_cast<int*>(aligned(workspace));
+  uint8_t* w = aligned(workspace) + ALIGN;
   Head* h = reinterpret_cast<Head*>(w);
   uint8_t* dc = w + p.head;
   uint8_t* dm = ROWS ? dc : dc + p.digits;
@@ -687,7 +698,7 @@ static int product(const uint8_t* G, int64_t M, int64_t N, const float* f, const
   ADX_LAUNCH_CHECK();
   digit_kernel<ROWS><<<(unsigned)(db < cap ? db : cap), 256, 0, st>>>(F, f, n_red, L, p.Lb, p.n_pass, p.n_blk, h, dc, dm);
   ADX_LAUNCH_CHECK();
-  const Args a{G, M, N, dc, dm, L, p.Lb, p.n_pass, p.n_blk, p.tiles, p.n_split, p.nstage, sc, sm, &h->err, polls};
+  const Args a{G, M, N, dc, dm, L, p.Lb, p.n_pass, p.n_blk, p.tiles, p.n_split, p.nstage, sc, sm, &h->err, sticky, polls};
   const bool al = (N & 15) == 0 && (reinterpret_cast<uintptr_t>(G) & 15) == 0;
   const int rc = al ? launch<ROWS, true>(a, st) : launch<ROWS, false>(a, st);
   if (rc) return rc;
@@ -731,6 +742,17 @@ extern "C" int adx_rsvd_cols(const uint8_t* G, int64_t M, int64_t N, const float
   const int rc = rt::product<false>(G, M, N, f, Y, L, accumulate, Z, workspace, workspace_bytes, as_stream(stream));
   if (rc == ADX_ERR_WORKSPACE) adx_set_message("adx_rsvd_cols: workspace too small");
   return rc;
+}
+
+extern "C" int adx_rsvd_status(void* workspace, size_t workspace_bytes, int* status, void* stream) {
+  if (!workspace || !status) { adx_set_message("adx_rsvd_status: null pointer"); return ADX_ERR_ARG; }
+  if (workspace_bytes < 2 * rt::ALIGN) { adx_set_message("adx_rsvd_status: workspace too small"); return ADX_ERR_WORKSPACE; }
+  cudaStream_t st = as_stream(stream);
+  int* word = reinterpret_cast<int*>(rt::aligned(workspace));
+  ADX_CUDA_TRY(cudaMemcpyAsync(status, word, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ADX_CUDA_TRY(cudaStreamSynchronize(st));
+  ADX_CUDA_TRY(cudaMemsetAsync(word, 0, sizeof(int), st));
+  return ADX_OK;
 }
 
 extern "C" int adx_rsvd_wait_selftest(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* F, int L,

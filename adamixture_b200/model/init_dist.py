@@ -47,12 +47,18 @@ class CudaInitBackend:
     def rsvd_cols(self, G, f, B, M_local):
         from .. import ops
 
-        return ops.rsvd_cols(G, f.to(torch.float32).contiguous(), B, M_local)
+        ws = ops.rsvd_workspace(G.device, M_local, G.shape[1], B.shape[1])
+        out = ops.rsvd_cols(G, f.to(torch.float32).contiguous(), B, M_local, ws=ws)
+        ops.rsvd_check(ws)
+        return out
 
     def rsvd_rows(self, G, f, Y, M_local):
         from .. import ops
 
-        return ops.rsvd_rows(G, f.to(torch.float32).contiguous(), Y, M_local)
+        ws = ops.rsvd_workspace(G.device, M_local, G.shape[1], Y.shape[1])
+        out = ops.rsvd_rows(G, f.to(torch.float32).contiguous(), Y, M_local, ws=ws)
+        ops.rsvd_check(ws)
+        return out
 
     def bvls(self, A, B, lower, upper):
         from .. import ops

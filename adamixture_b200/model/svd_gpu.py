@@ -42,13 +42,16 @@ def _SVD_gpu_once(G, N, M, f, k, seed, power, tol, device):
     gen.manual_seed(seed)
     f = f.to(device=device, dtype=torch.float32).contiguous()
     proj = torch.randn((M, L), dtype=torch.float32, generator=gen, device=device)
-    accum = ops.rsvd_cols(G, f, proj, M)                       # prime pass: X' Omega
+    ws = ops.rsvd_workspace(G.device, M, N, L)
+    accum = ops.rsvd_cols(G, f, proj, M, ws=ws)                # prime pass: X' Omega
+    ops.rsvd_check(ws)
     orth, _, _ = eigSVD_gpu(accum.T)
     alpha = torch.tensor(0.0, device=device)
     singular = torch.zeros(L, device=device)
     for i in range(power):
-        ops.rsvd_rows(G, f, orth, M, out=proj)                 # proj = X orth
-        ops.rsvd_cols(G, f, proj, M, out=accum)                # accum = X' proj
+        ops.rsvd_rows(G, f, orth, M, out=proj, ws=ws)          # proj = X orth
+        ops.rsvd_cols(G, f, proj, M, out=accum, ws=ws)         # accum = X' proj
+        ops.rsvd_check(ws)
         Qm, S, _ = eigSVD_gpu(accum.sub(orth, alpha=alpha.item()).T)
         if i > 0:
             s_cur = S + alpha
@@ -62,7 +65,8 @@ def _SVD_gpu_once(G, N, M, f, k, seed, power, tol, device):
         if S[-1] > alpha:
             alpha = 0.5 * (S[-1] + alpha)
         orth.copy_(Qm)
-    ops.rsvd_rows(G, f, orth, M, out=proj)                     # final projection
+    ops.rsvd_rows(G, f, orth, M, out=proj, ws=ws)              # final projection
+    ops.rsvd_check(ws)
     u_c, s_all, v_c = eigSVD_gpu(proj.T)
     S_final = s_all[:k].contiguous()
     U_final = u_c[:, :k].contiguous()

@@ -205,8 +205,10 @@ def m_step_P(G, Q: torch.Tensor, M: int) -> torch.Tensor:
     Qf = Q.float().contiguous()
     zero = torch.zeros(M, dtype=torch.float32, device=Q.device)
     half = torch.full((M,), 0.5, dtype=torch.float32, device=Q.device)
-    num = ops.rsvd_rows(G, zero, Qf, M).double()          # sum over observed of g Q
-    shifted = ops.rsvd_rows(G, half, Qf, M).double()      # sum over observed of (g - 1) Q
+    ws = ops.rsvd_workspace(G.device, M, *Qf.shape)
+    num = ops.rsvd_rows(G, zero, Qf, M, ws=ws).double()   # sum over observed of g Q
+    shifted = ops.rsvd_rows(G, half, Qf, M, ws=ws).double()   # sum over observed of (g - 1) Q
+    ops.rsvd_check(ws)
     den = 2.0 * (num - shifted)                            # 2 sum over observed of Q
     return (num / den.clamp_min(1e-12)).clamp(1e-5, 1.0 - 1e-5)
 

@@ -477,30 +477,56 @@ def register_reference_ops() -> None:
 
 # ---------------------------------------------------------------- initialisation
 
-def _rsvd_workspace(device: torch.device, M: int, N: int, L: int) -> torch.Tensor:
-    """Scratch of one product, the call's own (the caching allocator keeps it to the current
-    stream), so products on several streams or threads do not share it."""
-    return torch.empty(query_size("adx_rsvd_workspace_bytes", M, N, L), dtype=torch.uint8, device=device)
+def rsvd_workspace(device: torch.device, M: int, N: int, L: int) -> torch.Tensor:
+    """Scratch for ``rsvd_rows`` / ``rsvd_cols`` of this shape, status word cleared: for a
+    caller that runs several products in turn on one stream and reads their status
+    (``rsvd_check``)."""
+    ws = torch.empty(query_size("adx_rsvd_workspace_bytes", M, N, L), dtype=torch.uint8, device=device)
+    ws[:512].zero_()
+    return ws
+
+
+def rsvd_check(ws: torch.Tensor) -> None:
+    """Raise if a bounded wait of a product that used ``ws`` ran out since the last check (its
+    output is NaN then). Synchronises the current stream."""
+    import ctypes
+
+    out = ctypes.c_int(0)
+    call("adx_rsvd_status", ws.data_ptr(), ws.numel(), ctypes.addressof(out), _stream(ws.device))
+    if out.value:
+        raise RuntimeError(f"randomized-SVD product reported status {out.value} (a bounded wait timed out)")
+
+
+def _rsvd_scratch(ws: torch.Tensor | None, device: torch.device, M: int, N: int, L: int) -> torch.Tensor:
+    """The caller's workspace, or one of the call's own (the caching allocator keeps it to the
+    current stream), so products on several streams or threads do not share it."""
+    if ws is None:
+        return torch.empty(query_size("adx_rsvd_workspace_bytes", M, N, L), dtype=torch.uint8, device=device)
+    _check(ws, "ws", torch.uint8, device)
+    return ws
 
 
 def rsvd_rows(G: torch.Tensor, f: torch.Tensor, B: torch.Tensor, M: int,
-              out: torch.Tensor | None = None) -> torch.Tensor:
-    """``Xc @ B`` for the centred genotypes (float32 ``[M, L]``), B float32 ``[N, L]``."""
+              out: torch.Tensor | None = None, ws: torch.Tensor | None = None) -> torch.Tensor:
+    """``Xc @ B`` for the centred genotypes (float32 ``[M, L]``), B float32 ``[N, L]``. ``ws``:
+    scratch from ``rsvd_workspace``, whose status the caller can read (``rsvd_check``)."""
     _check(G, "G", torch.uint8)
     _check(f, "f", torch.float32, G.device)
     _check(B, "B", torch.float32, G.device)
     N, L = B.shape
     Y = torch.empty((M, L), dtype=torch.float32, device=G.device) if out is None else out
     _check(Y, "out", torch.float32, G.device)
-    ws = _rsvd_workspace(G.device, M, N, L)
+    ws = _rsvd_scratch(ws, G.device, M, N, L)
     call("adx_rsvd_rows_ws", G.data_ptr(), M, N, f.data_ptr(), B.data_ptr(), L, Y.data_ptr(),
          ws.data_ptr(), ws.numel(), _stream(G.device))
     return Y
 
 
 def rsvd_cols(G: torch.Tensor, f: torch.Tensor, Y: torch.Tensor, M: int,
-              out: torch.Tensor | None = None, accumulate: bool = False) -> torch.Tensor:
-    """``Xc.T @ Y`` (float32 ``[N, L]``; added to ``out`` when ``accumulate``)."""
+              out: torch.Tensor | None = None, accumulate: bool = False,
+              ws: torch.Tensor | None = None) -> torch.Tensor:
+    """``Xc.T @ Y`` (float32 ``[N, L]``; added to ``out`` when ``accumulate``). ``ws``: as for
+    ``rsvd_rows``."""
     _check(G, "G", torch.uint8)
     _check(f, "f", torch.float32, G.device)
     _check(Y, "Y", torch.float32, G.device)
@@ -508,7 +534,7 @@ def rsvd_cols(G: torch.Tensor, f: torch.Tensor, Y: torch.Tensor, M: int,
     L = Y.shape[1]
     Z = torch.empty((N, L), dtype=torch.float32, device=G.device) if out is None else out
     _check(Z, "out", torch.float32, G.device)
-    ws = _rsvd_workspace(G.device, M, N, L)
+    ws = _rsvd_scratch(ws, G.device, M, N, L)
     call("adx_rsvd_cols", G.data_ptr(), M, N, f.data_ptr(), Y.data_ptr(), L, int(bool(accumulate)),
          Z.data_ptr(), ws.data_ptr(), ws.numel(), _stream(G.device))
     return Z

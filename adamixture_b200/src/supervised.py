@@ -49,8 +49,10 @@ def init_p_supervised_gpu(G: torch.Tensor, y: np.ndarray, K: int, M: int, eps: f
     B = torch.from_numpy(ind).to(G.device)
     zero = torch.zeros(M, dtype=torch.float32, device=G.device)
     half = torch.full((M,), 0.5, dtype=torch.float32, device=G.device)
-    num = ops.rsvd_rows(G, zero, B, M).double()           # sum of g over observed labelled
-    den = 2.0 * (num - ops.rsvd_rows(G, half, B, M).double())   # 2 x observed labelled
+    ws = ops.rsvd_workspace(G.device, M, N, K)
+    num = ops.rsvd_rows(G, zero, B, M, ws=ws).double()    # sum of g over observed labelled
+    den = 2.0 * (num - ops.rsvd_rows(G, half, B, M, ws=ws).double())   # 2 x observed labelled
+    ops.rsvd_check(ws)
     P = torch.where(den > 0, num / den.clamp_min(1e-300), torch.full_like(num, 0.5))
     return P.clamp(eps, 1.0 - eps)
 

@@ -268,6 +268,11 @@ int adx_rsvd_rows_ws(const uint8_t* G, int64_t M, int64_t N, const float* f, con
 int adx_rsvd_cols(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* Y, int L,
                   int accumulate, float* Z, void* workspace, size_t workspace_bytes,
                   void* stream);
+/* Read and clear the status word of a workspace of these products: ADX_OK, or ADX_ERR_TIMEOUT if
+ * a bounded wait of any product since the last read ran out (that product's output is NaN).
+ * Products only ever set the word: zero the workspace before its first use to read it.
+ * Synchronises the stream. */
+int adx_rsvd_status(void* workspace, size_t workspace_bytes, int* status, void* stream);
 /* Self-test of these products' bounded waits: one product (cols = 0: rows, else cols) whose
  * waits each give up after `limit` polls (at most the products' own limit). Where one runs out
  * the kernel ends by itself and every entry of `out` is NaN; limit = 0: every wait does. */

@@ -59,3 +59,48 @@ def test_a_wait_that_runs_out(ops, cols):
     assert bool(torch.isnan(out).all())
     assert torch.equal(product(G, f, F, M), before)
     assert np.isfinite(before.cpu().numpy()).all()
+
+
+def test_status_of_the_workspace(ops):
+    from adamixture_b200._lib import call
+
+    N, M, L = 300, 900, 4
+    G, f, X, gen = cohort(N, M, 5)
+    B = torch.randn((N, L), generator=gen, device="cuda")
+    ws = ops.rsvd_workspace(G.device, M, N, L)
+    out = ops.rsvd_rows(G, f, B, M, ws=ws)
+    ops.rsvd_check(ws)
+    call("adx_rsvd_wait_selftest", G.data_ptr(), M, N, f.data_ptr(), B.data_ptr(), L, 0, 0, torch.empty_like(out).data_ptr(),
+         ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(ops.rsvd_rows(G, f, B, M, ws=ws), out)   # a product of its own; the status stays
+    with pytest.raises(RuntimeError, match="status 5"):
+        ops.rsvd_check(ws)
+    ops.rsvd_check(ws)   # read once
+
+
+@pytest.mark.parametrize("caller", ["svd", "sharded", "frequencies", "supervised"])
+def test_callers_raise_on_a_timeout(ops, monkeypatch, caller):
+    # the word is set by hand in the workspaces that the callers make
+    from adamixture_b200.model.init_dist import CudaInitBackend
+    from adamixture_b200.model.svd_gpu import SVD_gpu
+    from adamixture_b200.model.warm_start import m_step_P
+    from adamixture_b200.src.supervised import init_p_supervised_gpu
+
+    N, M, K = 60, 200, 3
+    G, f, X, gen = cohort(N, M, 6)
+    Q = torch.rand((N, K), generator=gen, device="cuda")
+    run = {"svd": lambda: SVD_gpu(G, N, M, f, K, 1, 2, 1e-1, 256, G.device, 256),
+           "sharded": lambda: CudaInitBackend().rsvd_rows(G, f, Q, M),
+           "frequencies": lambda: m_step_P(G, Q, M),
+           "supervised": lambda: init_p_supervised_gpu(G, np.arange(N) % (K + 1), K, M)}[caller]
+    run()
+    plain = ops.rsvd_workspace
+
+    def timed_out(*args):
+        ws = plain(*args)
+        ws[:4].copy_(torch.tensor([5, 0, 0, 0], dtype=torch.uint8))
+        return ws
+
+    monkeypatch.setattr(ops, "rsvd_workspace", timed_out)
+    with pytest.raises(RuntimeError, match="status 5"):
+        run()

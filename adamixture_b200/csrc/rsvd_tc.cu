@@ -13,11 +13,23 @@
 // factor is taken to 31-bit fixed point relative to its column's largest magnitude and split
 // into four signed 8-bit digits (columns 4 x L of the B operand); products and sums are
 // exact in int32 (at most 3 x 128 x 4 Mi per digit and CTA), the CTAs' parts add exactly in
-// int64, and one rounding to float32 ends it. What is left is the quantization, at most 2^-31
-// of the column's largest magnitude per entry: 128 times finer than float32's own
-// rounding there. Against float64 the relative error is 2.5e-8 (the final rounding) where
-// float32 FMAs gave 5.6e-6 (N=100,000 x M=300,000). Columns with an infinity or a NaN, and SNPs with such
-// a frequency, are summed entry by entry in float32 instead (finalize kernels).
+// int64, and one rounding to float32 ends it. What is left is the quantization: per entry at
+// most 2^-30 of the column's largest magnitude, 64 times finer than float32's own rounding
+// there (cols: the same of the codes' and of the flags' factor, the latter up to 3 times as
+// large). Against float64 the relative error is 2.5e-8 (the final rounding) where float32 FMAs
+// gave 5.6e-6 (N=100,000 x M=300,000).
+//
+// That error is the same for every entry of a column, so an output that meets small entries
+// only can be less exact than float32 FMAs make it. Per output both errors are sums: of n_S met
+// entries with the root mean square s they are about 2^-31 top sqrt(n_S) here and 2^-26 s n_S for
+// FMAs, so this form is the finer one from s = 2^-5 top / sqrt(n_S) on. A column is called wide
+// when more than 1/16 of its entries are inexact and below 2^-k of its largest magnitude, k = 4 +
+// log2(n) / 2 at most 8 (a Gaussian column has 2 % there, one carried by a few samples nearly
+// all). Wide columns take a second level, the same product with the remainders in 31 further
+// bits, which keeps all bits of entries down to 2^-37 of the largest: a CTA walks its range
+// twice when a column of its pass is wide. Columns that are wide once more (beyond 2^-31), that
+// hold an infinity or a NaN, and SNPs with such a frequency, are summed entry by entry in
+// float32 (finalize kernels).
 //
 // CTA: 256 rows of the product (two 128-row MMA tiles) over a range of 256-entry blocks of
 // the contracted axis. Rows are SNPs and the contraction runs over samples, or the reverse:
@@ -32,8 +44,9 @@
 // columns of a pass, is at most 24 so that two A stages fit; a wider factor takes
 // ceil(L / 24) passes of equal width.
 //
-// One pass each way at N=100,000 x M=300,000, L=20: 120.3 ms on float32 CUDA cores, 11.5 ms
-// here (the packed matrix read twice is 2.3 ms of HBM time).
+// One pass each way at N=100,000 x M=300,000, L=20: 120.3 ms on float32 CUDA cores, 11.6 ms
+// here (the packed matrix read twice is 2.3 ms of HBM time). Wide columns: N = M = 100,000, a
+// product 2.0 -> 3.9 ms (21 and 35 on the CUDA cores).
 // What bounds it now is the hand-over of the A stages: with no MMAs issued the loop still takes
 // 60 % of the time, and each MMA adds the 50 cycles that it takes; the time does not depend on
 // L (16 to 24), nor on the loads, nor on the unpacking itself.
@@ -82,11 +95,15 @@ static_assert(3ll * 128 * MAX_RED < (1ll << 31), "int32 digit sums");
 static_assert(2 * 2 * NDIG * LB_MAX + NSTAGE_MIN * 64 <= 512, "accumulators and the A stages in tensor memory");
 static_assert(G_ROW % 16 == 0 && G_BYTES % 16 == 0, "16-byte copies");
 
+struct Head;
+
 struct Args {
   const uint8_t* G;
   int64_t M, N;
   const uint8_t* dc;       // digit tiles of the codes' factor: [pass][block][256 x 4 Lb bytes]
   const uint8_t* dm;       // of the flags' factor (rows: the same tiles)
+  size_t level_bytes;      // from the first level's digits (dc, dm) to the second's
+  int64_t level_sums;      // and of the sums (sc, sm)
   int L, Lb, n_pass;
   int64_t n_blk;           // contracted blocks
   int64_t tiles;           // row tiles of 256
@@ -94,6 +111,7 @@ struct Args {
   int nstage;
   long long* sc;           // [rows][L] code sums (rows: S1 - 3 S2)
   long long* sm;           // [rows][L] flag sums
+  const Head* head;
   int* err;                // status of this product
   int* sticky;             // and of the workspace, until it is read
   uint32_t polls;          // limit of a wait
@@ -235,6 +253,21 @@ __device__ __forceinline__ uint32_t row_offset(const Args& a, int lr) {
   return ((uint32_t)(reinterpret_cast<uintptr_t>(a.G) & 15) + (uint32_t)lr * (uint32_t)(a.N & 15)) & 15u;
 }
 
+// Head of the workspace: the quanta (0: a column of zeros, or not finite), constant sums of the
+// two levels, entries that the levels hold too coarsely, what follows from them, status. The first
+// kernel of a product clears it.
+constexpr int N_FACT = 3;       // factors: of the codes, of the flags, of the constant sum
+constexpr int LEVELS = 2;
+constexpr int WIDE = 1, DIRECT = 2;
+struct Head {
+  double quantum[N_FACT][L_MAX];
+  unsigned long long csum[LEVELS][L_MAX];
+  unsigned long long coarse[LEVELS][L_MAX];
+  int mode[L_MAX];                // of a column: 0, WIDE (takes the second level), + DIRECT (float32)
+  int wide[L_MAX / LB_MAX + 1];   // a column of the pass is WIDE
+  int err;
+};
+
 template <bool ROWS, bool AL>
 __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -265,9 +298,13 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_holder)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  const int levels = a.head->wide[pass] ? LEVELS : 1;
+  for (int level = 0; level < levels; ++level) {
   if (tid == 0) {
     *abort_flag = 0;
     *joined = 0;
+    if (level)   // the barriers of the first level, all complete
+      for (int s = 0; s < N_BARS; ++s) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bars + 8u * (uint32_t)s) : "memory");
     for (int s = 0; s < NSLOT; ++s) {
       // 32 asynchronous and 32 plain arrivals of the load warp, and the bulk copies' expect
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 65;" ::"r"(FULL(s)));
@@ -293,7 +330,7 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
       const int64_t blk = q0 + q;
       if (lane == 0) {
         arrive_expect(FULL(slot), (ROWS ? 1u : 2u) * dbytes);
-        const int64_t at = ((int64_t)pass * a.n_blk + blk) * dbytes;
+        const int64_t at = ((int64_t)pass * a.n_blk + blk) * dbytes + level * a.level_bytes;
         bulk_copy(smem_u32(gs + G_BYTES), a.dc + at, dbytes, FULL(slot));
         if constexpr (!ROWS) bulk_copy(smem_u32(gs + G_BYTES + dbytes), a.dm + at, dbytes, FULL(slot));
       }
@@ -411,7 +448,8 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
     }
   }
   warp_wait(DONE, 0u, abort_flag, a.polls);
-  if (__syncthreads_or(*abort_flag)) {
+  const bool gave_up = __syncthreads_or(*abort_flag);
+  if (gave_up) {
     // a wait ran out: before the block ends, the copies and MMAs in flight land (these waits are
     // bounded too)
     if (tid == 0) {
@@ -453,8 +491,8 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
             for (int d = NDIG - 2; d >= 0; --d) s[o] = s[o] * 256 + (int)v[o][d][e];
           }
           if (ROWS) s[0] -= 3 * s[1];
-          if (row < n_rows && lg < a.L) {
-            const int64_t w = row * a.L + lg;
+          if (row < n_rows && lg < a.L && (!level || (a.head->mode[lg] & WIDE))) {
+            const int64_t w = level * a.level_sums + row * a.L + lg;
             if (a.n_split == 1) {
               a.sc[w] = s[0];
               a.sm[w] = s[1];
@@ -470,8 +508,10 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
   fence_before();
   __syncthreads();
   fence_after();
+  if (gave_up) break;
+  }
   if (warp == MMA_WARP) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(*tmem_holder));
   }
 }
 
@@ -485,91 +525,147 @@ __device__ __forceinline__ double factor(int which, float y, float f) {
   const double u = 2.0 * (double)f * (double)y;
   return which == 1 ? u - 3.0 * (double)y : u;
 }
-constexpr int N_FACT = 3;       // codes, flags, constant sum
-constexpr int SUM_BITS = 36;    // fixed point of the cols product's constant sum
+constexpr int BITS = 30;        // fixed point of the codes' and flags' factors
+constexpr int SUM_BITS = 36;    // and of the cols product's constant sum
+constexpr int LOW_BITS = 31;    // further bits of the second level
 
-// Head of the workspace: largest magnitudes (float bits), constant sums, status.
-struct Head {
-  uint32_t top[N_FACT][L_MAX];
-  unsigned long long csum[L_MAX];
-  int err;
-};
-
-// 2^bits over a power of two above the column's largest magnitude.
-__device__ __forceinline__ double quantum_inv(uint32_t top, int bits) {
-  return top ? ldexp(1.0, bits - 1 - ilogbf(__uint_as_float(top))) : 0.0;
-}
-__device__ __forceinline__ bool finite_bits(uint32_t top) { return top < 0x7F800000u; }
-
+// Largest magnitudes (float bits, which order as the magnitudes do, a NaN's above all) of a
+// block's entries per factor and column. The first block clears the head.
+constexpr int TOP_BLOCKS = 148;
 template <bool ROWS>
 __global__ void __launch_bounds__(256) top_kernel(const float* __restrict__ F, const float* __restrict__ f, int64_t n,
-                                                  int L, Head* h) {
-  __shared__ uint32_t top[N_FACT][L_MAX];
-  for (int e = threadIdx.x; e < N_FACT * L_MAX; e += 256) top[e / L_MAX][e % L_MAX] = 0;
+                                                  int L, Head* h, uint32_t* __restrict__ tops) {
+  constexpr int W = ROWS ? 1 : N_FACT;
+  __shared__ uint32_t top[W][L_MAX];
+  if (blockIdx.x == 0)
+    for (int e = threadIdx.x; e < (int)(sizeof(Head) / 4); e += 256) reinterpret_cast<uint32_t*>(h)[e] = 0;
+  for (int e = threadIdx.x; e < W * L_MAX; e += 256) top[e / L_MAX][e % L_MAX] = 0;
   __syncthreads();
   const int per = 256 / L, l = threadIdx.x % L, g = threadIdx.x / L;
   if (g < per) {
-    uint32_t t[N_FACT] = {0, 0, 0};
-    for (int64_t i = (int64_t)blockIdx.x * per + g; i < n; i += (int64_t)gridDim.x * per) {
-      const float y = F[i * L + l], fi = ROWS ? 0.0f : f[i];
-      // the magnitudes' bits order as the magnitudes do, a NaN's above all
+    uint32_t t[W] = {};
+    constexpr int U = 8;   // entries in flight
+    const int64_t step = (int64_t)gridDim.x * per;
+    for (int64_t i0 = (int64_t)blockIdx.x * per + g; i0 < n; i0 += U * step) {
+      float y[U], fi[U];
 #pragma unroll
-      for (int w = 0; w < (ROWS ? 1 : N_FACT); ++w)
-        t[w] = max(t[w], __float_as_uint((float)factor<ROWS>(w, y, fi)) & 0x7FFFFFFFu);
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = i0 + u * step;
+        y[u] = i < n ? F[i * L + l] : 0.0f;
+        fi[u] = !ROWS && i < n ? f[i] : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+          t[w] = max(t[w], __float_as_uint((float)factor<ROWS>(w, y[u], fi[u])) & 0x7FFFFFFFu);
     }
 #pragma unroll
-    for (int w = 0; w < (ROWS ? 1 : N_FACT); ++w) atomicMax(&top[w][l], t[w]);
+    for (int w = 0; w < W; ++w) atomicMax(&top[w][l], t[w]);
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < (ROWS ? 1 : N_FACT) * L; e += 256)
-    atomicMax(&h->top[e / L][e % L], top[e / L][e % L]);
+  for (int e = threadIdx.x; e < W * L; e += 256) tops[(int64_t)blockIdx.x * W * L + e] = top[e / L][e % L];
 }
 
-// Thread per (16 contracted entries, factor column): 16 bytes of each digit, in the order of
-// the shared-memory tile (32-entry steps of 4 Lb x 32 bytes: core matrices of 8 columns x 16
-// entries). Entries past n and columns past L are zero.
-template <bool ROWS>
+// Thread per (16 contracted entries, factor column): 16 bytes of each digit of a level, in the
+// order of the shared-memory tile (32-entry steps of 4 Lb x 32 bytes: core matrices of 8
+// columns x 16 entries). Entries past n and columns past L are zero. LOW: the second level, whose
+// launch does nothing when no column is wide.
+template <bool ROWS, bool LOW>
 __global__ void __launch_bounds__(256) digit_kernel(const float* __restrict__ F, const float* __restrict__ f,
                                                     int64_t n, int L, int Lb, int n_pass, int64_t n_blk, Head* h,
+                                                    const uint32_t* __restrict__ tops, int n_tops,
                                                     uint8_t* __restrict__ dc, uint8_t* __restrict__ dm) {
+  constexpr int W = ROWS ? 1 : N_FACT;
   __shared__ unsigned long long csum[L_MAX];
-  for (int e = threadIdx.x; e < L_MAX; e += 256) csum[e] = 0;
+  __shared__ uint32_t coarse[L_MAX], top[W * L_MAX];
+  __shared__ double per_quantum[W][L_MAX];   // 0: the column has no digits
+  if (LOW && !__syncthreads_or(threadIdx.x < n_pass && h->wide[threadIdx.x])) return;
+  for (int e = threadIdx.x; e < L_MAX; e += 256) { csum[e] = 0; coarse[e] = 0; }
+  if constexpr (!LOW) {
+    for (int e = threadIdx.x; e < W * L; e += 256) top[e] = 0;
+    __syncthreads();
+    const int groups = max(1, 256 / (W * L)), part = threadIdx.x / (W * L);
+    if (part < groups)
+      for (int e = threadIdx.x - part * W * L; e < W * L; e += 256) {
+        uint32_t t = 0;
+        for (int b = part; b < n_tops; b += 16 * groups) {
+          uint32_t v[16];
+#pragma unroll
+          for (int u = 0; u < 16; ++u) v[u] = b + u * groups < n_tops ? tops[(b + u * groups) * W * L + e] : 0u;
+#pragma unroll
+          for (int u = 0; u < 16; ++u) t = max(t, v[u]);
+        }
+        atomicMax(&top[e], t);
+      }
+  }
   __syncthreads();
+  if (threadIdx.x < L) {
+    const int l = threadIdx.x;
+    bool on = true;
+    if constexpr (LOW) {
+      on = (h->mode[l] & WIDE) != 0;
+    } else {
+#pragma unroll
+      for (int w = 0; w < W; ++w) on = on && top[w * L + l] < 0x7F800000u;
+      if (!on && blockIdx.x == 0) atomicOr(&h->mode[l], DIRECT);
+    }
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      // a quantum is 2^-bits of a power of two above the largest magnitude
+      double inv = 0.0;
+      if constexpr (LOW) {
+        if (on && h->quantum[w][l] > 0.0) inv = 1.0 / h->quantum[w][l];
+      } else {
+        const uint32_t t = top[w * L + l];
+        if (on && t) inv = ldexp(1.0, (w == 2 ? SUM_BITS : BITS) - 1 - ilogbf(__uint_as_float(t)));
+        if (blockIdx.x == 0) h->quantum[w][l] = inv > 0.0 ? 1.0 / inv : 0.0;
+      }
+      per_quantum[w][l] = inv;
+    }
+  }
+  __syncthreads();
+  // entries below `small` (the largest is at least 2^29) are below 2^-k of the largest
+  const int k = 4 + min(4, (63 - __clzll(n)) / 2);
+  const double low = (double)(1u << LOW_BITS), small = (double)(1 << (BITS - k)) / (LOW ? low : 1.0);
   const int cols = n_pass * Lb;
   const int64_t work = n_blk * (BLK / 16) * cols;
   for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < work; e += (int64_t)gridDim.x * 256) {
     const int64_t kg = e / cols;
     const int lg = (int)(e - kg * cols), pass = lg / Lb, lc = lg - pass * Lb;
-    const bool on = lg < L && finite_bits(h->top[0][lg]) && (ROWS || (finite_bits(h->top[1][lg]) && finite_bits(h->top[2][lg])));
-    double inv[N_FACT] = {0.0, 0.0, 0.0};
-    if (on) {
-      inv[0] = quantum_inv(h->top[0][lg], 30);
-      if (!ROWS) {
-        inv[1] = quantum_inv(h->top[1][lg], 30);
-        inv[2] = quantum_inv(h->top[2][lg], SUM_BITS);
-      }
-    }
-    long long c = 0;
-    uint32_t dig[2][NDIG][4] = {};
+    double inv[W] = {};
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int64_t i = kg * 16 + k;
+    for (int w = 0; w < W; ++w) inv[w] = lg < L ? per_quantum[w][lg] : 0.0;
+    const bool on = inv[0] > 0.0;   // else y is 0 throughout, or the column is not taken
+    long long c = 0;
+    uint32_t n_coarse = 0, dig[2][NDIG][4] = {};
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int64_t i = kg * 16 + u;
       const bool in = on && i < n;
       const float y = in ? F[i * L + lg] : 0.0f, fi = !ROWS && in ? f[i] : 0.0f;
+      bool lost = false;
 #pragma unroll
-      for (int w = 0; w < (ROWS ? 1 : 2); ++w) {
-        int q = __double2int_rn(factor<ROWS>(w, y, fi) * inv[w]);
-        if (ROWS) c += q;
+      for (int w = 0; w < W; ++w) {
+        const double x = factor<ROWS>(w, y, fi) * inv[w];
+        const double r = LOW ? (x - rint(x)) * low : x;   // the difference is exact
+        const double qr = rint(r);
+        lost = lost || (qr != r && fabs(x) < small);
+        if (ROWS || w == 2) c += (long long)qr;
+        if (w < 2) {
+          int q = (int)qr;
 #pragma unroll
-        for (int d = 0; d < NDIG; ++d) {
-          const int lo = (int)(int8_t)(q & 0xFF);   // signed digit; the rest divides exactly
-          dig[w][d][k >> 2] |= (uint32_t)(lo & 0xFF) << (8 * (k & 3));
-          q = (q - lo) >> 8;
+          for (int d = 0; d < NDIG; ++d) {
+            const int lo = (int)(int8_t)(q & 0xFF);   // signed digit; the rest divides exactly
+            dig[w][d][u >> 2] |= (uint32_t)(lo & 0xFF) << (8 * (u & 3));
+            q = (q - lo) >> 8;
+          }
         }
       }
-      if (!ROWS) c += __double2ll_rn(factor<ROWS>(2, y, fi) * inv[2]);
+      n_coarse += lost;
     }
     if (on) atomicAdd(&csum[lg], (unsigned long long)c);
+    if (n_coarse) atomicAdd(&coarse[lg], n_coarse);
     const int64_t base = ((int64_t)pass * n_blk * (BLK / 32) + (kg >> 1)) * (32 * NDIG * Lb);
 #pragma unroll
     for (int d = 0; d < NDIG; ++d) {
@@ -580,43 +676,62 @@ __global__ void __launch_bounds__(256) digit_kernel(const float* __restrict__ F,
     }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < L; e += 256)
-    if (csum[e]) atomicAdd(&h->csum[e], csum[e]);
+  for (int e = threadIdx.x; e < L; e += 256) {
+    if (csum[e]) atomicAdd(&h->csum[LOW][e], csum[e]);
+    // the block whose entries bring the count past n / 16 says so
+    if (coarse[e] && 16 * (int64_t)(atomicAdd(&h->coarse[LOW][e], (unsigned long long)coarse[e]) + coarse[e]) > n) {
+      atomicOr(&h->mode[e], LOW ? DIRECT : WIDE);
+      if (!LOW) h->wide[e / Lb] = 1;
+    }
+  }
+}
+
+// Output (row, l) entry by entry in float32.
+template <bool ROWS>
+__device__ __noinline__ float direct(const uint8_t* __restrict__ G, int64_t N, const float* __restrict__ F,
+                                     const float* __restrict__ f, int L, int64_t n_red, int64_t row, int l) {
+  float v = 0.0f;
+#pragma unroll 8
+  for (int64_t r = 0; r < n_red; ++r) {
+    const int64_t j = ROWS ? row : r, i = ROWS ? r : row;
+    const unsigned g = genotype(__ldg(G + (j >> 2) * N + i), (int)(j & 3));
+    const float x = g == 3u ? 0.0f : (float)g - 2.0f * __ldg(f + j);
+    v = fmaf(x, __ldg(F + r * L + l), v);
+  }
+  return v;
 }
 
 // One thread per output element: the integer sums to float32. Elements whose factor column
-// or frequency is not finite are summed directly, as float32 arithmetic would have them.
+// or frequency is not finite, or whose column is wider than both levels, are summed directly, as
+// float32 arithmetic has them.
 template <bool ROWS>
 __global__ void __launch_bounds__(256) finalize_kernel(const uint8_t* __restrict__ G, int64_t M, int64_t N,
                                                        const float* __restrict__ F, const float* __restrict__ f, int L,
                                                        const long long* __restrict__ sc,
-                                                       const long long* __restrict__ sm, const Head* __restrict__ h,
-                                                       int accumulate, float* __restrict__ out) {
+                                                       const long long* __restrict__ sm, int64_t level_sums,
+                                                       const Head* __restrict__ h, int accumulate,
+                                                       float* __restrict__ out) {
+  const int64_t n_rows = ROWS ? M : N, n_red = ROWS ? N : M;
   const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  const int64_t n_rows = ROWS ? M : N;
   if (e >= n_rows * L) return;
   const int64_t row = e / L;
   const int l = (int)(e - row * L);
-  const uint32_t t0 = h->top[0][l], t1 = h->top[1][l], t2 = h->top[2][l];
   const float fr = ROWS ? f[row] : 0.0f;
   float v;
   if (h->err) {
     v = __uint_as_float(0x7FFFFFFFu);   // a bounded wait ran out: not a result
-  } else if (!finite_bits(t0) || !finite_bits(t1) || !finite_bits(t2) || (ROWS && !isfinite(fr))) {
-    v = 0.0f;
-    for (int64_t r = 0; r < (ROWS ? N : M); ++r) {
-      const int64_t j = ROWS ? row : r, i = ROWS ? r : row;
-      const unsigned g = genotype(G[(j >> 2) * N + i], (int)(j & 3));
-      const float x = g == 3u ? 0.0f : (float)g - 2.0f * f[j];
-      v = fmaf(x, F[r * L + l], v);
-    }
-  } else if (ROWS) {
-    const double q = t0 ? 1.0 / quantum_inv(t0, 30) : 0.0;
-    v = (float)(q * ((double)sc[e] - 2.0 * (double)fr * (double)((long long)h->csum[l] - sm[e])));
+  } else if ((h->mode[l] & DIRECT) || (ROWS && !isfinite(fr))) {
+    v = direct<ROWS>(G, N, F, f, L, n_red, row, l);
   } else {
-    const double q0 = t0 ? 1.0 / quantum_inv(t0, 30) : 0.0, q1 = t1 ? 1.0 / quantum_inv(t1, 30) : 0.0;
-    const double q2 = t2 ? 1.0 / quantum_inv(t2, SUM_BITS) : 0.0;
-    v = (float)(q0 * (double)sc[e] + q1 * (double)sm[e] - q2 * (double)(long long)h->csum[l]);
+    auto sum = [&](int u) {
+      const int64_t at = u * level_sums + e;
+      const long long cs = (long long)h->csum[u][l];
+      return ROWS ? h->quantum[0][l] * ((double)sc[at] - 2.0 * (double)fr * (double)(cs - sm[at]))
+                  : h->quantum[0][l] * (double)sc[at] + h->quantum[1][l] * (double)sm[at] - h->quantum[2][l] * (double)cs;
+    };
+    double t = sum(0);
+    if (h->mode[l] & WIDE) t += sum(1) * (1.0 / (double)(1u << LOW_BITS));
+    v = (float)t;
   }
   out[e] = accumulate ? out[e] + v : v;
 }
@@ -628,7 +743,7 @@ constexpr size_t ALIGN = 256;   // of the workspace's parts (bulk copies read fr
 struct Plan {
   int Lb, n_pass, n_split, nstage;
   int64_t n_blk, tiles;
-  size_t head, digits, sums, bytes;   // bytes of each part and in all
+  size_t head, tops, digits, sums, bytes;   // bytes of each part and in all
 };
 
 // Splits of the contracted axis: the count whose CTAs (one per SM) finish first, counting
@@ -653,9 +768,10 @@ static Plan plan(int64_t n_rows, int64_t n_red, int L, bool rows) {
   }
   auto pad = [](size_t b) { return (b + ALIGN - 1) & ~(ALIGN - 1); };
   p.head = pad(sizeof(Head));
+  p.tops = pad((size_t)TOP_BLOCKS * (rows ? 1 : N_FACT) * L * sizeof(uint32_t));
   p.digits = pad((size_t)p.n_pass * p.n_blk * digit_bytes(p.Lb));
   p.sums = pad((size_t)n_rows * L * sizeof(long long));
-  p.bytes = ALIGN + p.head + (rows ? 1 : 2) * p.digits + 2 * p.sums + ALIGN;
+  p.bytes = ALIGN + p.head + p.tops + LEVELS * ((rows ? 1 : 2) * p.digits + 2 * p.sums) + ALIGN;
   return p;
 }
 
@@ -686,23 +802,32 @@ static int product(const uint8_t* G, int64_t M, int64_t N, const float* f, const
   int* sticky = reinterpret_cast<int*>(aligned(workspace));
   uint8_t* w = aligned(workspace) + ALIGN;
   Head* h = reinterpret_cast<Head*>(w);
-  uint8_t* dc = w + p.head;
+  uint32_t* tops = reinterpret_cast<uint32_t*>(w + p.head);
+  uint8_t* dc = w + p.head + p.tops;
   uint8_t* dm = ROWS ? dc : dc + p.digits;
-  long long* sc = reinterpret_cast<long long*>(dm + p.digits);
+  const size_t level_bytes = (ROWS ? 1 : 2) * p.digits;
+  long long* sc = reinterpret_cast<long long*>(dc + LEVELS * level_bytes);
   long long* sm = reinterpret_cast<long long*>(reinterpret_cast<uint8_t*>(sc) + p.sums);
-  ADX_CUDA_TRY(cudaMemsetAsync(h, 0, sizeof(Head), st));
-  if (p.n_split > 1) ADX_CUDA_TRY(cudaMemsetAsync(sc, 0, 2 * p.sums, st));
+  const int64_t level_sums = 2 * (int64_t)(p.sums / sizeof(long long));
+  if (p.n_split > 1) ADX_CUDA_TRY(cudaMemsetAsync(sc, 0, LEVELS * 2 * p.sums, st));
   const int64_t cap = (int64_t)sm_count() * 8;
   const int64_t tb = ceil_div(n_red, 8 * (256 / L)), db = ceil_div(p.n_blk * (BLK / 16) * p.n_pass * p.Lb, 256);
-  top_kernel<ROWS><<<(unsigned)(tb < cap ? tb : cap), 256, 0, st>>>(F, f, n_red, L, h);
+  const int n_tops = (int)(tb < TOP_BLOCKS ? tb : TOP_BLOCKS);
+  top_kernel<ROWS><<<n_tops, 256, 0, st>>>(F, f, n_red, L, h, tops);
   ADX_LAUNCH_CHECK();
-  digit_kernel<ROWS><<<(unsigned)(db < cap ? db : cap), 256, 0, st>>>(F, f, n_red, L, p.Lb, p.n_pass, p.n_blk, h, dc, dm);
+  digit_kernel<ROWS, false><<<(unsigned)(db < cap ? db : cap), 256, 0, st>>>(F, f, n_red, L, p.Lb, p.n_pass, p.n_blk, h, tops,
+                                                                           n_tops, dc, dm);
   ADX_LAUNCH_CHECK();
-  const Args a{G, M, N, dc, dm, L, p.Lb, p.n_pass, p.n_blk, p.tiles, p.n_split, p.nstage, sc, sm, &h->err, sticky, polls};
+  digit_kernel<ROWS, true><<<(unsigned)(db < cap / 4 ? db : cap / 4), 256, 0, st>>>(
+      F, f, n_red, L, p.Lb, p.n_pass, p.n_blk, h, tops, n_tops, dc + level_bytes, dm + level_bytes);
+  ADX_LAUNCH_CHECK();
+  const Args a{G, M, N, dc, dm, level_bytes, level_sums, L, p.Lb, p.n_pass, p.n_blk, p.tiles, p.n_split,
+               p.nstage, sc, sm, h, &h->err, sticky, polls};
   const bool al = (N & 15) == 0 && (reinterpret_cast<uintptr_t>(G) & 15) == 0;
   const int rc = al ? launch<ROWS, true>(a, st) : launch<ROWS, false>(a, st);
   if (rc) return rc;
-  finalize_kernel<ROWS><<<(unsigned)ceil_div(n_rows * L, 256), 256, 0, st>>>(G, M, N, F, f, L, sc, sm, h, accumulate, out);
+  finalize_kernel<ROWS><<<(unsigned)ceil_div(n_rows * L, 256), 256, 0, st>>>(G, M, N, F, f, L, sc, sm, level_sums,
+                                                                                  h, accumulate, out);
   ADX_LAUNCH_CHECK();
   return ADX_OK;
 }

@@ -508,8 +508,9 @@ def _rsvd_scratch(ws: torch.Tensor | None, device: torch.device, M: int, N: int,
 
 def rsvd_rows(G: torch.Tensor, f: torch.Tensor, B: torch.Tensor, M: int,
               out: torch.Tensor | None = None, ws: torch.Tensor | None = None) -> torch.Tensor:
-    """``Xc @ B`` for the centred genotypes (float32 ``[M, L]``), B float32 ``[N, L]``. ``ws``:
-    scratch from ``rsvd_workspace``, whose status the caller can read (``rsvd_check``)."""
+    """``Xc @ B`` for the centred genotypes (float32 ``[M, L]``), B float32 ``[N, L]``. Columns
+    whose entries spread widely (more than 1/16 of them below 2^-8 of the largest) take twice the
+    time. ``ws``: scratch from ``rsvd_workspace``, whose status the caller can read (``rsvd_check``)."""
     _check(G, "G", torch.uint8)
     _check(f, "f", torch.float32, G.device)
     _check(B, "B", torch.float32, G.device)

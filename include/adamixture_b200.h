@@ -260,7 +260,8 @@ int adx_rsvd_rows(const uint8_t* G, int64_t M, int64_t N, const float* f, const 
                   float* Y, void* stream);
 int adx_rsvd_workspace_bytes(int64_t M, int64_t N, int L, size_t* bytes);
 /* The same with a workspace (adx_rsvd_workspace_bytes, any alignment): on the integer tensor
- * cores, from the factor in 31-bit fixed point. */
+ * cores, from the factor in 31-bit fixed point relative to its column's largest magnitude; 62 bits
+ * for columns whose entries spread widely (at twice the time), float32 beyond that. */
 int adx_rsvd_rows_ws(const uint8_t* G, int64_t M, int64_t N, const float* f, const float* B, int L,
                      float* Y, void* workspace, size_t workspace_bytes, void* stream);
 /* Z[N][L] = Xc' Y (accumulate != 0: Z += Xc' Y), Y float32 [M][L]; on the integer tensor

@@ -27,9 +27,10 @@
 // log2(n) / 2 at most 8 (a Gaussian column has 2 % there, one carried by a few samples nearly
 // all). Wide columns take a second level, the same product with the remainders in 31 further
 // bits, which keeps all bits of entries down to 2^-37 of the largest: a CTA walks its range
-// twice when a column of its pass is wide. Columns that are wide once more (beyond 2^-31), that
-// hold an infinity or a NaN, and SNPs with such a frequency, are summed entry by entry in
-// float32 (finalize kernels).
+// twice when a column of its pass is wide. Columns that are wide once more (beyond 2^-31) and
+// SNPs whose frequency is not finite (rows) are summed entry by entry in float32, in turn
+// (finalize kernels). Infinite and NaN entries of the factor, and of f (cols), have no digits:
+// their terms are added in float32 at the end.
 //
 // CTA: 256 rows of the product (two 128-row MMA tiles) over a range of 256-entry blocks of
 // the contracted axis. Rows are SNPs and the contraction runs over samples, or the reverse:
@@ -253,18 +254,22 @@ __device__ __forceinline__ uint32_t row_offset(const Args& a, int lr) {
   return ((uint32_t)(reinterpret_cast<uintptr_t>(a.G) & 15) + (uint32_t)lr * (uint32_t)(a.N & 15)) & 15u;
 }
 
-// Head of the workspace: the quanta (0: a column of zeros, or not finite), constant sums of the
-// two levels, entries that the levels hold too coarsely, what follows from them, status. The first
-// kernel of a product clears it.
+// Head of the workspace: the quanta (0: a column of zeros), constant sums of the two levels,
+// entries that the levels hold too coarsely, what follows from them, entries without digits,
+// status. The first kernel of a product clears it.
 constexpr int N_FACT = 3;       // factors: of the codes, of the flags, of the constant sum
 constexpr int LEVELS = 2;
-constexpr int WIDE = 1, DIRECT = 2;
+constexpr int WIDE = 1, DIRECT = 2, ODD = 4;   // takes the second level; summed directly; has entries without digits
+constexpr int MAX_ODD = 64;     // entries added one by one; with more, their columns are summed directly
 struct Head {
   double quantum[N_FACT][L_MAX];
   unsigned long long csum[LEVELS][L_MAX];
   unsigned long long coarse[LEVELS][L_MAX];
-  int mode[L_MAX];                // of a column: 0, WIDE (takes the second level), + DIRECT (float32)
+  int mode[L_MAX];                // of a column: bits
   int wide[L_MAX / LB_MAX + 1];   // a column of the pass is WIDE
+  int n_odd;                      // entries without digits, the first MAX_ODD of them
+  int64_t odd_row[MAX_ODD];
+  int odd_col[MAX_ODD];
   int err;
 };
 
@@ -525,13 +530,27 @@ __device__ __forceinline__ double factor(int which, float y, float f) {
   const double u = 2.0 * (double)f * (double)y;
   return which == 1 ? u - 3.0 * (double)y : u;
 }
+// Their magnitudes as float bits, which order as the magnitudes do (float32 rounds them; the digits
+// have room for that). An entry with one that is not finite has no digits.
+template <bool ROWS>
+__device__ __forceinline__ bool magnitudes(float y, float f, uint32_t (&t)[ROWS ? 1 : N_FACT]) {
+  t[0] = __float_as_uint(y) & 0x7FFFFFFFu;
+  if constexpr (!ROWS) {
+    t[1] = __float_as_uint((2.0f * f - 3.0f) * y) & 0x7FFFFFFFu;
+    t[2] = __float_as_uint(2.0f * f * y) & 0x7FFFFFFFu;
+  }
+  uint32_t top = t[0];
+#pragma unroll
+  for (int w = 1; w < (ROWS ? 1 : N_FACT); ++w) top = max(top, t[w]);
+  return top < 0x7F800000u;
+}
 constexpr int BITS = 30;        // fixed point of the codes' and flags' factors
 constexpr int SUM_BITS = 36;    // and of the cols product's constant sum
 constexpr int LOW_BITS = 31;    // further bits of the second level
 
-// Largest magnitudes (float bits, which order as the magnitudes do, a NaN's above all) of a
-// block's entries per factor and column. The first block clears the head.
-constexpr int TOP_BLOCKS = 148;
+// Largest magnitudes of a block's entries per factor and column. The first block clears the head.
+constexpr int TOP_BLOCKS = 296;
+__host__ __device__ constexpr int top_stride(int w, int L) { return (w * L + 3) / 4 * 4; }   // 16-byte loads
 template <bool ROWS>
 __global__ void __launch_bounds__(256) top_kernel(const float* __restrict__ F, const float* __restrict__ f, int64_t n,
                                                   int L, Head* h, uint32_t* __restrict__ tops) {
@@ -555,16 +574,19 @@ __global__ void __launch_bounds__(256) top_kernel(const float* __restrict__ F, c
         fi[u] = !ROWS && i < n ? f[i] : 0.0f;
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u)
+      for (int u = 0; u < U; ++u) {
+        uint32_t m[W];
+        if (magnitudes<ROWS>(y[u], fi[u], m))
 #pragma unroll
-        for (int w = 0; w < W; ++w)
-          t[w] = max(t[w], __float_as_uint((float)factor<ROWS>(w, y[u], fi[u])) & 0x7FFFFFFFu);
+          for (int w = 0; w < W; ++w) t[w] = max(t[w], m[w]);
+      }
     }
 #pragma unroll
     for (int w = 0; w < W; ++w) atomicMax(&top[w][l], t[w]);
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < W * L; e += 256) tops[(int64_t)blockIdx.x * W * L + e] = top[e / L][e % L];
+  for (int e = threadIdx.x; e < top_stride(W, L); e += 256)
+    tops[blockIdx.x * top_stride(W, L) + e] = e < W * L ? top[e / L][e % L] : 0u;
 }
 
 // Thread per (16 contracted entries, factor column): 16 bytes of each digit of a level, in the
@@ -572,44 +594,45 @@ __global__ void __launch_bounds__(256) top_kernel(const float* __restrict__ F, c
 // columns x 16 entries). Entries past n and columns past L are zero. LOW: the second level, whose
 // launch does nothing when no column is wide.
 template <bool ROWS, bool LOW>
-__global__ void __launch_bounds__(256) digit_kernel(const float* __restrict__ F, const float* __restrict__ f,
+__global__ void __launch_bounds__(256, 3) digit_kernel(const float* __restrict__ F, const float* __restrict__ f,
                                                     int64_t n, int L, int Lb, int n_pass, int64_t n_blk, Head* h,
                                                     const uint32_t* __restrict__ tops, int n_tops,
                                                     uint8_t* __restrict__ dc, uint8_t* __restrict__ dm) {
   constexpr int W = ROWS ? 1 : N_FACT;
   __shared__ unsigned long long csum[L_MAX];
-  __shared__ uint32_t coarse[L_MAX], top[W * L_MAX];
+  __shared__ uint32_t coarse[L_MAX];
+  __shared__ __align__(16) uint32_t top[top_stride(W, L_MAX)];
   __shared__ double per_quantum[W][L_MAX];   // 0: the column has no digits
   if (LOW && !__syncthreads_or(threadIdx.x < n_pass && h->wide[threadIdx.x])) return;
   for (int e = threadIdx.x; e < L_MAX; e += 256) { csum[e] = 0; coarse[e] = 0; }
   if constexpr (!LOW) {
-    for (int e = threadIdx.x; e < W * L; e += 256) top[e] = 0;
+    const int quads = top_stride(W, L) / 4, groups = 256 / quads, part = threadIdx.x / quads;
+    const int e = 4 * (threadIdx.x - part * quads);
+    if (part == 0) *reinterpret_cast<uint4*>(top + e) = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    const int groups = max(1, 256 / (W * L)), part = threadIdx.x / (W * L);
-    if (part < groups)
-      for (int e = threadIdx.x - part * W * L; e < W * L; e += 256) {
-        uint32_t t = 0;
-        for (int b = part; b < n_tops; b += 16 * groups) {
-          uint32_t v[16];
+    if (part < groups) {
+      uint4 t = make_uint4(0u, 0u, 0u, 0u);
+      constexpr int U = 8;   // loads in flight
+      for (int b = part; b < n_tops; b += U * groups) {
+        uint4 v[U];
 #pragma unroll
-          for (int u = 0; u < 16; ++u) v[u] = b + u * groups < n_tops ? tops[(b + u * groups) * W * L + e] : 0u;
+        for (int u = 0; u < U; ++u)
+          v[u] = b + u * groups < n_tops ? *reinterpret_cast<const uint4*>(tops + (b + u * groups) * 4 * quads + e)
+                                         : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-          for (int u = 0; u < 16; ++u) t = max(t, v[u]);
-        }
-        atomicMax(&top[e], t);
+        for (int u = 0; u < U; ++u)
+          t = make_uint4(max(t.x, v[u].x), max(t.y, v[u].y), max(t.z, v[u].z), max(t.w, v[u].w));
       }
+      atomicMax(top + e, t.x);
+      atomicMax(top + e + 1, t.y);
+      atomicMax(top + e + 2, t.z);
+      atomicMax(top + e + 3, t.w);
+    }
   }
   __syncthreads();
   if (threadIdx.x < L) {
     const int l = threadIdx.x;
-    bool on = true;
-    if constexpr (LOW) {
-      on = (h->mode[l] & WIDE) != 0;
-    } else {
-#pragma unroll
-      for (int w = 0; w < W; ++w) on = on && top[w * L + l] < 0x7F800000u;
-      if (!on && blockIdx.x == 0) atomicOr(&h->mode[l], DIRECT);
-    }
+    const bool on = !LOW || (h->mode[l] & WIDE);
 #pragma unroll
     for (int w = 0; w < W; ++w) {
       // a quantum is 2^-bits of a power of two above the largest magnitude
@@ -618,7 +641,7 @@ __global__ void __launch_bounds__(256) digit_kernel(const float* __restrict__ F,
         if (on && h->quantum[w][l] > 0.0) inv = 1.0 / h->quantum[w][l];
       } else {
         const uint32_t t = top[w * L + l];
-        if (on && t) inv = ldexp(1.0, (w == 2 ? SUM_BITS : BITS) - 1 - ilogbf(__uint_as_float(t)));
+        if (t) inv = ldexp(1.0, (w == 2 ? SUM_BITS : BITS) - 1 - ilogbf(__uint_as_float(t)));
         if (blockIdx.x == 0) h->quantum[w][l] = inv > 0.0 ? 1.0 / inv : 0.0;
       }
       per_quantum[w][l] = inv;
@@ -631,19 +654,29 @@ __global__ void __launch_bounds__(256) digit_kernel(const float* __restrict__ F,
   const int cols = n_pass * Lb;
   const int64_t work = n_blk * (BLK / 16) * cols;
   for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < work; e += (int64_t)gridDim.x * 256) {
-    const int64_t kg = e / cols;
+    const int64_t kg = work <= UINT32_MAX ? (uint32_t)e / (uint32_t)cols : e / cols;
     const int lg = (int)(e - kg * cols), pass = lg / Lb, lc = lg - pass * Lb;
     double inv[W] = {};
 #pragma unroll
     for (int w = 0; w < W; ++w) inv[w] = lg < L ? per_quantum[w][lg] : 0.0;
-    const bool on = inv[0] > 0.0;   // else y is 0 throughout, or the column is not taken
+    const bool on = lg < L && (!LOW || inv[0] > 0.0);
     long long c = 0;
     uint32_t n_coarse = 0, dig[2][NDIG][4] = {};
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
       const int64_t i = kg * 16 + u;
       const bool in = on && i < n;
-      const float y = in ? F[i * L + lg] : 0.0f, fi = !ROWS && in ? f[i] : 0.0f;
+      float y = in ? F[i * L + lg] : 0.0f, fi = !ROWS && in ? f[i] : 0.0f;
+      uint32_t m[W];
+      if (!magnitudes<ROWS>(y, fi, m)) {
+        if (!LOW) {
+          atomicOr(&h->mode[lg], ODD);
+          // counted until they are too many
+          const int at = *(volatile int*)&h->n_odd <= MAX_ODD ? atomicAdd(&h->n_odd, 1) : MAX_ODD;
+          if (at < MAX_ODD) { h->odd_row[at] = i; h->odd_col[at] = lg; }
+        }
+        y = fi = 0.0f;
+      }
       bool lost = false;
 #pragma unroll
       for (int w = 0; w < W; ++w) {
@@ -686,24 +719,40 @@ __global__ void __launch_bounds__(256) digit_kernel(const float* __restrict__ F,
   }
 }
 
-// Output (row, l) entry by entry in float32.
+// v + the term of contracted entry r in output (row, l), in float32.
+template <bool ROWS>
+__device__ __forceinline__ float term(const uint8_t* __restrict__ G, int64_t N, const float* __restrict__ F,
+                                      const float* __restrict__ f, int L, int64_t r, int64_t row, int l, float v) {
+  const int64_t j = ROWS ? row : r, i = ROWS ? r : row;
+  const unsigned g = genotype(__ldg(G + (j >> 2) * N + i), (int)(j & 3));
+  const float x = g == 3u ? 0.0f : (float)g - 2.0f * __ldg(f + j);
+  return fmaf(x, __ldg(F + r * L + l), v);
+}
+
+// Output (row, l) entry by entry; a NaN stays one.
 template <bool ROWS>
 __device__ __noinline__ float direct(const uint8_t* __restrict__ G, int64_t N, const float* __restrict__ F,
                                      const float* __restrict__ f, int L, int64_t n_red, int64_t row, int l) {
   float v = 0.0f;
-#pragma unroll 8
-  for (int64_t r = 0; r < n_red; ++r) {
-    const int64_t j = ROWS ? row : r, i = ROWS ? r : row;
-    const unsigned g = genotype(__ldg(G + (j >> 2) * N + i), (int)(j & 3));
-    const float x = g == 3u ? 0.0f : (float)g - 2.0f * __ldg(f + j);
-    v = fmaf(x, __ldg(F + r * L + l), v);
-  }
+  int64_t r = 0;
+  for (; r + 8 <= n_red && v == v; r += 8)
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v = term<ROWS>(G, N, F, f, L, r + u, row, l, v);
+  for (; r < n_red && v == v; ++r) v = term<ROWS>(G, N, F, f, L, r, row, l, v);
   return v;
 }
 
-// One thread per output element: the integer sums to float32. Elements whose factor column
-// or frequency is not finite, or whose column is wider than both levels, are summed directly, as
-// float32 arithmetic has them.
+// v + the terms of the entries without digits.
+template <bool ROWS>
+__device__ __noinline__ float add_odd(const uint8_t* __restrict__ G, int64_t N, const float* __restrict__ F,
+                                      const float* __restrict__ f, int L, const Head* __restrict__ h, int64_t row, int l,
+                                      float v) {
+  for (int k = 0; k < h->n_odd; ++k)
+    if (h->odd_col[k] == l) v = term<ROWS>(G, N, F, f, L, h->odd_row[k], row, l, v);
+  return v;
+}
+
+// One thread per output element: the integer sums to float32.
 template <bool ROWS>
 __global__ void __launch_bounds__(256) finalize_kernel(const uint8_t* __restrict__ G, int64_t M, int64_t N,
                                                        const float* __restrict__ F, const float* __restrict__ f, int L,
@@ -714,13 +763,14 @@ __global__ void __launch_bounds__(256) finalize_kernel(const uint8_t* __restrict
   const int64_t n_rows = ROWS ? M : N, n_red = ROWS ? N : M;
   const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (e >= n_rows * L) return;
-  const int64_t row = e / L;
+  const int64_t row = n_rows * L <= UINT32_MAX ? (uint32_t)e / (uint32_t)L : e / L;
   const int l = (int)(e - row * L);
   const float fr = ROWS ? f[row] : 0.0f;
+  const int mode = h->mode[l];
   float v;
   if (h->err) {
     v = __uint_as_float(0x7FFFFFFFu);   // a bounded wait ran out: not a result
-  } else if ((h->mode[l] & DIRECT) || (ROWS && !isfinite(fr))) {
+  } else if ((mode & DIRECT) || ((mode & ODD) && h->n_odd > MAX_ODD) || (ROWS && !isfinite(fr))) {
     v = direct<ROWS>(G, N, F, f, L, n_red, row, l);
   } else {
     auto sum = [&](int u) {
@@ -730,8 +780,9 @@ __global__ void __launch_bounds__(256) finalize_kernel(const uint8_t* __restrict
                   : h->quantum[0][l] * (double)sc[at] + h->quantum[1][l] * (double)sm[at] - h->quantum[2][l] * (double)cs;
     };
     double t = sum(0);
-    if (h->mode[l] & WIDE) t += sum(1) * (1.0 / (double)(1u << LOW_BITS));
+    if (mode & WIDE) t += sum(1) * (1.0 / (double)(1u << LOW_BITS));
     v = (float)t;
+    if (mode & ODD) v = add_odd<ROWS>(G, N, F, f, L, h, row, l, v);
   }
   out[e] = accumulate ? out[e] + v : v;
 }
@@ -768,7 +819,7 @@ static Plan plan(int64_t n_rows, int64_t n_red, int L, bool rows) {
   }
   auto pad = [](size_t b) { return (b + ALIGN - 1) & ~(ALIGN - 1); };
   p.head = pad(sizeof(Head));
-  p.tops = pad((size_t)TOP_BLOCKS * (rows ? 1 : N_FACT) * L * sizeof(uint32_t));
+  p.tops = pad((size_t)TOP_BLOCKS * top_stride(rows ? 1 : N_FACT, L) * sizeof(uint32_t));
   p.digits = pad((size_t)p.n_pass * p.n_blk * digit_bytes(p.Lb));
   p.sums = pad((size_t)n_rows * L * sizeof(long long));
   p.bytes = ALIGN + p.head + p.tops + LEVELS * ((rows ? 1 : 2) * p.digits + 2 * p.sums) + ALIGN;

@@ -8,6 +8,7 @@ centred matrix of at most 2 (cols: codes, flags and constant, 8); then the round
 result to float32 and of the float64 sums that end it: cols adds three terms of up to 3 times
 the large entry that cancel, 2^-50 with room. Below that an entry is summed in float32: n
 roundings of 2^-24 of a partial sum. Float32 sums of entries at 2^-34 are bound to 2^-58 n^2 only."""
+import numpy as np
 import pytest
 import torch
 
@@ -75,3 +76,55 @@ def test_short_contractions(ops, n):
     mag = X.abs() @ F.double().abs()
     # no further off than float32 sums are bound to be
     assert bool(((got - ref).abs() <= 2.0 ** -24 * ((n + 1) * mag + ref.abs())).all())
+
+
+@pytest.mark.parametrize("bad", [1, 3, 70])
+@pytest.mark.parametrize("side", ["rows", "cols"])
+def test_entries_that_are_not_finite(ops, bad, side):
+    # few: added one by one; more than the list holds: every output in turn. In f (cols) a missing
+    # genotype keeps the SNP out of the sample's sum; in f (rows) the SNP's own outputs change
+    cols = side == "cols"
+    N, M, L = 257, 301, 5
+    n = M if cols else N
+    G, f, X, gen = cohort(N, M, bad, 2, cols)
+    product = ops.rsvd_cols if cols else ops.rsvd_rows
+    F = torch.randn((n, L), generator=gen, device="cuda")
+    at = torch.randperm(n, generator=gen, device="cuda")[:bad]
+    F[at, 1] = float("inf")
+    F[at[:1], 2] = float("nan")
+    F[at, 3] = torch.where(torch.arange(bad, device="cuda") % 2 == 0, float("inf"), -float("inf"))
+    got = product(G, f, F, M)
+    A = X.T if cols else X
+    ref = (A[:, :, None] * F.double()[None]).sum(1)
+    clean = ref.isfinite()
+    assert torch.equal(got[~clean], ref[~clean].float()) or torch.equal(got.isnan(), ref.isnan())
+    assert torch.equal(got.isposinf(), ref.isposinf()) and torch.equal(got.isneginf(), ref.isneginf())
+    assert bool(((got - ref).abs()[clean] <= 2.0 ** -22 * (A.abs() @ F.double().abs().nan_to_num(0, 0, 0))[clean]).all())
+
+    f[at] = float("nan")   # rows: `at` as SNPs
+    F = torch.randn((n, L), generator=gen, device="cuda")
+    got = product(G, f, F, M)
+    miss = (X == 0) & torch.from_numpy(unpack(G, M) == 3).cuda()
+    Xn = torch.where(miss, 0.0, (X + 0.0 * f.double()[:, None]))
+    A = Xn.T if cols else Xn
+    ref = (A[:, :, None] * F.double()[None]).sum(1)
+    assert torch.equal(got.isnan(), ref.isnan())
+    fine = ~ref.isnan()
+    assert bool(((got - ref).abs()[fine] <= 2.0 ** -22 * (A.abs() @ F.double().abs())[fine]).all())
+
+
+def unpack(G, M):
+    g = G.cpu().numpy()
+    return np.stack([g >> (2 * s) & 3 for s in range(4)], 1).reshape(-1, g.shape[1])[:M]
+
+
+def test_a_column_of_nans_leaves_the_others_alone(ops):
+    N, M, L = 300, 400, 4
+    G, f, X, gen = cohort(N, M, 8, 2, False)
+    B = torch.randn((N, L), generator=gen, device="cuda")
+    Y = torch.randn((M, L), generator=gen, device="cuda")
+    plain = ops.rsvd_rows(G, f, B, M), ops.rsvd_cols(G, f, Y, M)
+    B[:, 2] = Y[:, 2] = float("nan")
+    for got, ref in zip((ops.rsvd_rows(G, f, B, M), ops.rsvd_cols(G, f, Y, M)), plain):
+        assert bool(got[:, 2].isnan().all())
+        assert torch.equal(got[:, [0, 1, 3]], ref[:, [0, 1, 3]])

@@ -12,7 +12,7 @@
 // and every sum over the matrix is one of small integers (c, m) times a factor column. The
 // factor is taken to 31-bit fixed point relative to its column's largest magnitude and split
 // into four signed 8-bit digits (columns 4 x L of the B operand); products and sums are
-// exact in int32 (at most 3 x 128 x 4 Mi per digit and CTA), the CTAs' parts add exactly in
+// exact in int32 (at most 3 x 128 x 0.5 Mi per digit and CTA), the CTAs' parts add exactly in
 // int64, and one rounding to float32 ends it. What is left is the quantization: per entry at
 // most 2^-30 of the column's largest magnitude, 64 times finer than float32's own rounding
 // there (cols: the same of the codes' and of the flags' factor, the latter up to 3 times as
@@ -55,6 +55,8 @@
 
 #include <math.h>
 
+#include <algorithm>
+
 namespace adx {
 namespace rt {
 
@@ -90,9 +92,14 @@ constexpr int G_ROW = BLK + 16;           // bytes of a packed row in a slot, an
 constexpr int G_BYTES = (OWN / 4) * G_ROW;
 constexpr int N_BARS = 2 * NSLOT + NSTAGE_MAX + 1;
 constexpr uint32_t POLLS = 1u << 22;      // of a bounded wait: a fraction of a second to a few seconds
-constexpr int64_t MAX_RED = int64_t(1) << 22;   // contracted entries per CTA: int32 sums are exact
+// A launch takes at most so many row tiles and contracted blocks, so that the workspace stays
+// bounded (32 bytes an output, at most 16 L a contracted entry): 606,208 rows, 16 full rounds of
+// CTAs, and 524,288 contracted entries. At L=20 that is 0.39 GB at most; one launch for all
+// would take 6.4 GB for 10 million SNPs.
+constexpr int64_t MAX_TILES = 148 * 16, MAX_BLOCKS = 2048;
+static_assert(MAX_TILES * OWN * L_MAX < (1ll << 32), "32-bit output indices");
 static_assert(OWN == BLK, "a block of G has the same shape in both products");
-static_assert(3ll * 128 * MAX_RED < (1ll << 31), "int32 digit sums");
+static_assert(3ll * 128 * MAX_BLOCKS * BLK < (1ll << 31), "int32 digit sums");
 static_assert(2 * 2 * NDIG * LB_MAX + NSTAGE_MIN * 64 <= 512, "accumulators and the A stages in tensor memory");
 static_assert(G_ROW % 16 == 0 && G_BYTES % 16 == 0, "16-byte copies");
 
@@ -106,12 +113,13 @@ struct Args {
   size_t level_bytes;      // from the first level's digits (dc, dm) to the second's
   int64_t level_sums;      // and of the sums (sc, sm)
   int L, Lb, n_pass;
-  int64_t n_blk;           // contracted blocks
-  int64_t tiles;           // row tiles of 256
+  int64_t blk0, n_blk;     // contracted blocks
+  int64_t tile0, tiles;    // row tiles of 256
   int n_split;             // ranges of the contracted axis
   int nstage;
-  long long* sc;           // [rows][L] code sums (rows: S1 - 3 S2)
-  long long* sm;           // [rows][L] flag sums
+  bool add;                // to the sums (several ranges or launches), else they are written
+  long long* sc;           // [rows of the tiles][L] code sums (rows: S1 - 3 S2)
+  long long* sm;           // [rows of the tiles][L] flag sums
   const Head* head;
   int* err;                // status of this product
   int* sticky;             // and of the workspace, until it is read
@@ -292,7 +300,7 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
   volatile int* joined = reinterpret_cast<volatile int*>(ctl + 8 * N_BARS + 8);   // stages the MMA warp has passed
 
   int64_t b = blockIdx.x;
-  const int64_t tile = b % a.tiles; b /= a.tiles;
+  const int64_t tile = a.tile0 + b % a.tiles; b /= a.tiles;
   const int split = (int)(b % a.n_split);
   const int pass = (int)(b / a.n_split);
   const int64_t per = (a.n_blk + a.n_split - 1) / a.n_split;
@@ -332,10 +340,10 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
     for (int q = 0; q < nq; ++q) {
       if (fill > 0 && !warp_wait(EMPTY(slot), (fill - 1) & 1u, abort_flag, a.polls)) break;
       uint8_t* gs = sm + slot * slot_bytes;
-      const int64_t blk = q0 + q;
+      const int64_t blk = a.blk0 + q0 + q;
       if (lane == 0) {
         arrive_expect(FULL(slot), (ROWS ? 1u : 2u) * dbytes);
-        const int64_t at = ((int64_t)pass * a.n_blk + blk) * dbytes + level * a.level_bytes;
+        const int64_t at = ((int64_t)pass * a.n_blk + q0 + q) * dbytes + level * a.level_bytes;
         bulk_copy(smem_u32(gs + G_BYTES), a.dc + at, dbytes, FULL(slot));
         if constexpr (!ROWS) bulk_copy(smem_u32(gs + G_BYTES + dbytes), a.dm + at, dbytes, FULL(slot));
       }
@@ -497,8 +505,8 @@ __global__ void __launch_bounds__(TPB, 1) product_kernel(Args a) {
           }
           if (ROWS) s[0] -= 3 * s[1];
           if (row < n_rows && lg < a.L && (!level || (a.head->mode[lg] & WIDE))) {
-            const int64_t w = level * a.level_sums + row * a.L + lg;
-            if (a.n_split == 1) {
+            const int64_t w = level * a.level_sums + (row - a.tile0 * OWN) * a.L + lg;
+            if (!a.add) {
               a.sc[w] = s[0];
               a.sm[w] = s[1];
             } else {   // integers: the order does not matter
@@ -591,11 +599,14 @@ __global__ void __launch_bounds__(256) top_kernel(const float* __restrict__ F, c
 
 // Thread per (16 contracted entries, factor column): 16 bytes of each digit of a level, in the
 // order of the shared-memory tile (32-entry steps of 4 Lb x 32 bytes: core matrices of 8
-// columns x 16 entries). Entries past n and columns past L are zero. LOW: the second level, whose
-// launch does nothing when no column is wide.
+// columns x 16 entries), for n_blk blocks from blk0. Entries past n and columns past L are zero.
+// LOW: the second level, whose launch does nothing when no column is wide. does: COUNT (constant
+// sums, coarse and odd entries), WRITE (digits).
+constexpr int COUNT = 1, WRITE = 2;
 template <bool ROWS, bool LOW>
 __global__ void __launch_bounds__(256, 3) digit_kernel(const float* __restrict__ F, const float* __restrict__ f,
-                                                    int64_t n, int L, int Lb, int n_pass, int64_t n_blk, Head* h,
+                                                    int64_t n, int L, int Lb, int n_pass, int64_t blk0,
+                                                    int64_t n_blk, int does, Head* h,
                                                     const uint32_t* __restrict__ tops, int n_tops,
                                                     uint8_t* __restrict__ dc, uint8_t* __restrict__ dm) {
   constexpr int W = ROWS ? 1 : N_FACT;
@@ -664,12 +675,12 @@ __global__ void __launch_bounds__(256, 3) digit_kernel(const float* __restrict__
     uint32_t n_coarse = 0, dig[2][NDIG][4] = {};
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
-      const int64_t i = kg * 16 + u;
+      const int64_t i = blk0 * BLK + kg * 16 + u;
       const bool in = on && i < n;
       float y = in ? F[i * L + lg] : 0.0f, fi = !ROWS && in ? f[i] : 0.0f;
       uint32_t m[W];
       if (!magnitudes<ROWS>(y, fi, m)) {
-        if (!LOW) {
+        if (!LOW && (does & COUNT)) {
           atomicOr(&h->mode[lg], ODD);
           // counted until they are too many
           const int at = *(volatile int*)&h->n_odd <= MAX_ODD ? atomicAdd(&h->n_odd, 1) : MAX_ODD;
@@ -699,6 +710,7 @@ __global__ void __launch_bounds__(256, 3) digit_kernel(const float* __restrict__
     }
     if (on) atomicAdd(&csum[lg], (unsigned long long)c);
     if (n_coarse) atomicAdd(&coarse[lg], n_coarse);
+    if (!(does & WRITE)) continue;
     const int64_t base = ((int64_t)pass * n_blk * (BLK / 32) + (kg >> 1)) * (32 * NDIG * Lb);
 #pragma unroll
     for (int d = 0; d < NDIG; ++d) {
@@ -709,6 +721,7 @@ __global__ void __launch_bounds__(256, 3) digit_kernel(const float* __restrict__
     }
   }
   __syncthreads();
+  if (!(does & COUNT)) return;
   for (int e = threadIdx.x; e < L; e += 256) {
     if (csum[e]) atomicAdd(&h->csum[LOW][e], csum[e]);
     // the block whose entries bring the count past n / 16 says so
@@ -752,19 +765,20 @@ __device__ __noinline__ float add_odd(const uint8_t* __restrict__ G, int64_t N, 
   return v;
 }
 
-// One thread per output element: the integer sums to float32.
+// One thread per output element of `rows` rows from row0: the integer sums to float32.
 template <bool ROWS>
 __global__ void __launch_bounds__(256) finalize_kernel(const uint8_t* __restrict__ G, int64_t M, int64_t N,
+                                                       int64_t row0, int64_t rows,
                                                        const float* __restrict__ F, const float* __restrict__ f, int L,
                                                        const long long* __restrict__ sc,
                                                        const long long* __restrict__ sm, int64_t level_sums,
                                                        const Head* __restrict__ h, int accumulate,
                                                        float* __restrict__ out) {
-  const int64_t n_rows = ROWS ? M : N, n_red = ROWS ? N : M;
-  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (e >= n_rows * L) return;
-  const int64_t row = n_rows * L <= UINT32_MAX ? (uint32_t)e / (uint32_t)L : e / L;
-  const int l = (int)(e - row * L);
+  const int64_t n_red = ROWS ? N : M;
+  const uint32_t e = blockIdx.x * 256 + threadIdx.x;   // of at most MAX_TILES * OWN * L_MAX
+  if (e >= rows * L) return;
+  const int64_t row = row0 + e / (uint32_t)L;
+  const int l = (int)(e % (uint32_t)L);
   const float fr = ROWS ? f[row] : 0.0f;
   const int mode = h->mode[l];
   float v;
@@ -784,7 +798,8 @@ __global__ void __launch_bounds__(256) finalize_kernel(const uint8_t* __restrict
     v = (float)t;
     if (mode & ODD) v = add_odd<ROWS>(G, N, F, f, L, h, row, l, v);
   }
-  out[e] = accumulate ? out[e] + v : v;
+  float* o = out + row0 * L + e;
+  *o = accumulate ? *o + v : v;
 }
 
 // ---------------------------------------------------------------- plan
@@ -792,13 +807,11 @@ __global__ void __launch_bounds__(256) finalize_kernel(const uint8_t* __restrict
 constexpr size_t ALIGN = 256;   // of the workspace's parts (bulk copies read from it); any caller's pointer will do
 
 struct Plan {
-  int Lb, n_pass, n_split, nstage;
-  int64_t n_blk, tiles;
+  int Lb, n_pass, nstage;
+  int64_t n_blk, tiles;     // in all
   size_t head, tops, digits, sums, bytes;   // bytes of each part and in all
 };
 
-// Splits of the contracted axis: the count whose CTAs (one per SM) finish first, counting
-// blocks and about 3 blocks of prologue and epilogue per CTA; the smallest of equals.
 static Plan plan(int64_t n_rows, int64_t n_red, int L, bool rows) {
   Plan p{};
   p.n_pass = (L + LB_MAX - 1) / LB_MAX;
@@ -807,23 +820,28 @@ static Plan plan(int64_t n_rows, int64_t n_red, int L, bool rows) {
   p.tiles = ceil_div(n_rows, OWN);
   const int fit = (512 - 4 * NDIG * p.Lb) / 64;
   p.nstage = fit < NSTAGE_MAX ? fit : NSTAGE_MAX;
-  const int64_t sms = 148;
-  const int64_t lo = ceil_div(p.n_blk * BLK, MAX_RED);
-  const int64_t hi = p.n_blk < lo + 255 ? p.n_blk : lo + 255;
-  int64_t best = -1;
-  for (int64_t s = lo; s <= hi; ++s) {
-    const int64_t per = ceil_div(p.n_blk, s);
-    if (ceil_div(p.n_blk, per) != s) continue;   // the same ranges as a smaller count
-    const int64_t t = ceil_div(p.tiles * p.n_pass * s, sms) * (per + 3);
-    if (best < 0 || t < best) { best = t; p.n_split = (int)s; }
-  }
   auto pad = [](size_t b) { return (b + ALIGN - 1) & ~(ALIGN - 1); };
   p.head = pad(sizeof(Head));
   p.tops = pad((size_t)TOP_BLOCKS * top_stride(rows ? 1 : N_FACT, L) * sizeof(uint32_t));
-  p.digits = pad((size_t)p.n_pass * p.n_blk * digit_bytes(p.Lb));
-  p.sums = pad((size_t)n_rows * L * sizeof(long long));
+  p.digits = pad((size_t)p.n_pass * std::min(p.n_blk, MAX_BLOCKS) * digit_bytes(p.Lb));
+  p.sums = pad((size_t)std::min(n_rows, MAX_TILES * OWN) * L * sizeof(long long));
   p.bytes = ALIGN + p.head + p.tops + LEVELS * ((rows ? 1 : 2) * p.digits + 2 * p.sums) + ALIGN;
   return p;
+}
+
+// Splits of a launch's contracted axis: the count whose CTAs (one per SM) finish first, counting
+// blocks and about 3 blocks of prologue and epilogue per CTA; the smallest of equals.
+static int splits(int64_t tiles, int64_t n_blk, int n_pass) {
+  const int64_t sms = 148;
+  int64_t best = -1;
+  int n_split = 1;
+  for (int64_t s = 1; s <= std::min<int64_t>(n_blk, 256); ++s) {
+    const int64_t per = ceil_div(n_blk, s);
+    if (ceil_div(n_blk, per) != s) continue;   // the same ranges as a smaller count
+    const int64_t t = ceil_div(tiles * n_pass * s, sms) * (per + 3);
+    if (best < 0 || t < best) { best = t; n_split = (int)s; }
+  }
+  return n_split;
 }
 
 template <bool ROWS, bool AL>
@@ -860,26 +878,54 @@ static int product(const uint8_t* G, int64_t M, int64_t N, const float* f, const
   long long* sc = reinterpret_cast<long long*>(dc + LEVELS * level_bytes);
   long long* sm = reinterpret_cast<long long*>(reinterpret_cast<uint8_t*>(sc) + p.sums);
   const int64_t level_sums = 2 * (int64_t)(p.sums / sizeof(long long));
-  if (p.n_split > 1) ADX_CUDA_TRY(cudaMemsetAsync(sc, 0, LEVELS * 2 * p.sums, st));
-  const int64_t cap = (int64_t)sm_count() * 8;
-  const int64_t tb = ceil_div(n_red, 8 * (256 / L)), db = ceil_div(p.n_blk * (BLK / 16) * p.n_pass * p.Lb, 256);
+  const int64_t cap = (int64_t)sm_count() * 8, tb = ceil_div(n_red, 8 * (256 / L));
   const int n_tops = (int)(tb < TOP_BLOCKS ? tb : TOP_BLOCKS);
   top_kernel<ROWS><<<n_tops, 256, 0, st>>>(F, f, n_red, L, h, tops);
   ADX_LAUNCH_CHECK();
-  digit_kernel<ROWS, false><<<(unsigned)(db < cap ? db : cap), 256, 0, st>>>(F, f, n_red, L, p.Lb, p.n_pass, p.n_blk, h, tops,
-                                                                           n_tops, dc, dm);
-  ADX_LAUNCH_CHECK();
-  digit_kernel<ROWS, true><<<(unsigned)(db < cap / 4 ? db : cap / 4), 256, 0, st>>>(
-      F, f, n_red, L, p.Lb, p.n_pass, p.n_blk, h, tops, n_tops, dc + level_bytes, dm + level_bytes);
-  ADX_LAUNCH_CHECK();
-  const Args a{G, M, N, dc, dm, level_bytes, level_sums, L, p.Lb, p.n_pass, p.n_blk, p.tiles, p.n_split,
-               p.nstage, sc, sm, h, &h->err, sticky, polls};
+  auto digits = [&](int64_t blk0, int does) -> int {
+    const int64_t n_blk = std::min(p.n_blk - blk0, MAX_BLOCKS);
+    const int64_t db = ceil_div(n_blk * (BLK / 16) * p.n_pass * p.Lb, 256);
+    digit_kernel<ROWS, false><<<(unsigned)std::min(db, cap), 256, 0, st>>>(F, f, n_red, L, p.Lb, p.n_pass, blk0, n_blk, does, h,
+                                                                        tops, n_tops, dc, dm);
+    ADX_LAUNCH_CHECK();
+    return ADX_OK;
+  };
+  auto low_digits = [&](int64_t blk0, int does) -> int {
+    const int64_t n_blk = std::min(p.n_blk - blk0, MAX_BLOCKS);
+    const int64_t db = ceil_div(n_blk * (BLK / 16) * p.n_pass * p.Lb, 256);
+    digit_kernel<ROWS, true><<<(unsigned)std::min(db, cap / 4), 256, 0, st>>>(
+        F, f, n_red, L, p.Lb, p.n_pass, blk0, n_blk, does, h, tops, n_tops, dc + level_bytes, dm + level_bytes);
+    ADX_LAUNCH_CHECK();
+    return ADX_OK;
+  };
+  const bool several = p.n_blk > MAX_BLOCKS;   // the counts of all blocks come before the first product
+  int rc;
+  if (several) {
+    for (int64_t b = 0; b < p.n_blk; b += MAX_BLOCKS)
+      if ((rc = digits(b, COUNT))) return rc;
+    for (int64_t b = 0; b < p.n_blk; b += MAX_BLOCKS)
+      if ((rc = low_digits(b, COUNT))) return rc;
+  }
   const bool al = (N & 15) == 0 && (reinterpret_cast<uintptr_t>(G) & 15) == 0;
-  const int rc = al ? launch<ROWS, true>(a, st) : launch<ROWS, false>(a, st);
-  if (rc) return rc;
-  finalize_kernel<ROWS><<<(unsigned)ceil_div(n_rows * L, 256), 256, 0, st>>>(G, M, N, F, f, L, sc, sm, level_sums,
-                                                                                  h, accumulate, out);
-  ADX_LAUNCH_CHECK();
+  for (int64_t tile0 = 0; tile0 < p.tiles; tile0 += MAX_TILES) {
+    const int64_t tiles = std::min(p.tiles - tile0, MAX_TILES), row0 = tile0 * OWN, rows = std::min(n_rows - row0, tiles * OWN);
+    for (int64_t blk0 = 0; blk0 < p.n_blk; blk0 += MAX_BLOCKS) {
+      if (several || tile0 == 0) {   // else the digits stand
+        const int does = several ? WRITE : COUNT | WRITE;
+        if ((rc = digits(blk0, does)) || (rc = low_digits(blk0, does))) return rc;
+      }
+      const int64_t n_blk = std::min(p.n_blk - blk0, MAX_BLOCKS);
+      const int n_split = splits(tiles, n_blk, p.n_pass);
+      const bool add = several || n_split > 1;
+      if (add && blk0 == 0) ADX_CUDA_TRY(cudaMemsetAsync(sc, 0, LEVELS * 2 * p.sums, st));
+      const Args a{G, M, N, dc, dm, level_bytes, level_sums, L, p.Lb, p.n_pass, blk0, n_blk, tile0, tiles, n_split,
+                   p.nstage, add, sc, sm, h, &h->err, sticky, polls};
+      if ((rc = al ? launch<ROWS, true>(a, st) : launch<ROWS, false>(a, st))) return rc;
+    }
+    finalize_kernel<ROWS><<<(unsigned)ceil_div(rows * L, 256), 256, 0, st>>>(G, M, N, row0, rows, F, f, L, sc, sm, level_sums, h,
+                                                                           accumulate, out);
+    ADX_LAUNCH_CHECK();
+  }
   return ADX_OK;
 }
 

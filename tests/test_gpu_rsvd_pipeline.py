@@ -104,3 +104,26 @@ def test_callers_raise_on_a_timeout(ops, monkeypatch, caller):
     monkeypatch.setattr(ops, "rsvd_workspace", timed_out)
     with pytest.raises(RuntimeError, match="status 5"):
         run()
+
+
+# more rows and more contracted entries than one launch takes (606,208 and 524,288), with a last
+# launch that is nearly empty; one column wide, one with an infinity
+@pytest.mark.parametrize("N,M", [(9, 1_212_421), (524_300, 9), (606_209, 6)])
+def test_several_launches(ops, N, M):
+    L = 6
+    G, f, X, gen = cohort(N, M, N)
+    B = torch.randn((N, L), generator=gen, device="cuda")
+    Y = torch.randn((M, L), generator=gen, device="cuda")
+    for product, A, F in ((ops.rsvd_rows, X, B), (ops.rsvd_cols, X.T, Y)):
+        n = F.shape[0]
+        F[:, 1] *= 2.0 ** -20
+        F[n // 2, 1] = 1.0
+        F[n - 1, 2] = float("inf")
+        got, fine = product(G, f, F, M), [c for c in range(L) if c != 2]
+        ref = A @ F[:, fine].double()
+        tol = 8 * n * 2.0 ** -30 * F[:, fine].abs().amax(0).double() + 2.0 ** -23 * ref.abs()
+        assert bool(((got[:, fine].double() - ref).abs() <= tol).all())
+        assert bool((~got[:, 2].isfinite()).all())
+        once = product(G, f, F, M, out=torch.zeros_like(got)) if product is ops.rsvd_rows else \
+            product(G, f, F, M, out=torch.zeros_like(got), accumulate=True)
+        assert torch.equal(once[:, fine], got[:, fine])

@@ -395,8 +395,8 @@ __global__ void sqp_kernel(const double* __restrict__ H, const double* __restric
 // 0.61 ms here), so what counts is the latency of one iteration. Lane i holds row i of the tableau: the
 // parameters' columns, the constraint's (position KM), its last column (the step u_i) and
 // the last row's element i. A sweep on pivot k broadcasts p * tmp through shared memory and
-// is one multiply-add per element; every element sees the operations of sweep() above
-// in the same order, so the results are the same to the last bit.
+// is one multiply-add per element, the operations of sweep() above in the same order: in the
+// box, where both forms can solve the same problem, the results are equal to the last bit.
 template <int KM, bool SIMPLEX>
 struct RegTableau {
   static constexpr int C = KM + (SIMPLEX ? 1 : 0);   // parameters and the constraint

@@ -308,6 +308,8 @@ __device__ __forceinline__ float rcp(float x) {
   return r;
 }
 
+constexpr int ctas_per_sm(int K) { return K <= 2 ? 5 : K <= 4 ? 4 : K <= 6 ? 3 : 2; }   // registers without spills
+
 template <int K>
 struct Cfg {
   static constexpr int V = 2 * K;
@@ -317,7 +319,7 @@ struct Cfg {
   static constexpr int COLS = 4 * V4;                           // columns of a quad of SNPs
   static constexpr int LPC = COLS == 4 ? 8 : COLS == 8 ? 4 : 2; // lanes that share a column
   static constexpr int KP = (K + 1) / 2 * 2;                    // P row of a SNP: pairs {p, p}, 16-byte loads
-  static constexpr int OCC = K <= 2 ? 5 : K <= 4 ? 4 : K <= 6 ? 3 : 2;   // CTAs per SM: registers without spills
+  static constexpr int OCC = ctas_per_sm(K);
   static constexpr int CHK = K <= 6 ? 32 : 16;                  // SNPs per staged chunk (48 KB of shared memory)
 };
 
@@ -874,15 +876,21 @@ int em_plan(int64_t M, int64_t N, int K, int prec, EmPlan& pl) {
     n_mblk = ceil_div(M, mb);
   };
   blocks_of(PLAN_BLOCKS);
-  // Small cohorts (up to 2,048 samples): with PLAN_BLOCKS a CTA has one or a few chunks of SNPs,
-  // less than what its Q tile, its T partials and the pipeline's start cost (about 4 chunks of the
-  // float64 MMA form, 1 of the float32 pairs). Of 1 to 12 CTAs per SM (148, a constant, as above;
-  // 3 of the float32 form run at a time), the count whose CTAs finish first. At N=105 x M=8,451,
-  // K=7 in float64: 133 CTAs of 4 chunks in one round instead of 529 of one chunk in four.
+  // Small cohorts: with PLAN_BLOCKS a CTA has one or a few chunks of SNPs, less than what its Q
+  // tile, its T partials and the pipeline's start cost (about 4 chunks of the float64 MMA form, 1
+  // of the float32 pairs). Of 1 to 12 CTAs per SM (148, a constant, as above), the count whose
+  // CTAs finish first, as many at a time as the registers allow (float64: 1). At N=105 x
+  // M=8,451, K=7 in float64: 133 CTAs of 4 chunks in one round instead of 529 of one chunk in four.
+  // An iteration with PLAN_BLOCKS and with this rule: float64 K=10, 4,000 x 12,000 355 and 303 us,
+  // 4,000 x 30,000 (16 chunks and more: the rule does not apply) 772 both; from 4,096 samples the
+  // plan is left as it was. Float32 K=8, 5,000 x 30,000 527 and 402 us, 18,000 x 5,000 318 and 255;
+  // with K <= 4, whose chunks are short, 5,000 x 30,000 181 and 187, 16,000 x 30,000 536 and 517: no
+  // gain to speak of above 2,048 samples.
   const bool mma64 = prec == ADX_F64 && K <= DMMA_MAX_K, pairs32 = prec == ADX_F32 && K <= f32s::MAX_K;
   const int64_t own_tiles = ceil_div(pl.n_stile, n_split);
-  if ((mma64 || pairs32) && N <= 2048 && own_tiles * (mb / CH) < 16) {
-    const int64_t slots = mma64 ? 148 : 444, start = mma64 ? 4 : 1;
+  const int64_t most = mma64 ? 4095 : K <= 4 ? 2048 : 19999;
+  if ((mma64 || pairs32) && N <= most && own_tiles * (mb / CH) < 16) {
+    const int64_t slots = mma64 ? 148 : 148 * f32s::ctas_per_sm(K), start = mma64 ? 4 : 1;
     auto rounds = [&]() { return ceil_div(n_split * n_mblk, slots) * own_tiles * (mb / CH + start); };
     int64_t best = rounds(), best_blocks = PLAN_BLOCKS;
     for (int64_t blocks = PLAN_BLOCKS / slots * slots; blocks >= slots; blocks -= slots) {

@@ -639,13 +639,13 @@ __global__ void em_update_kernel(const R* __restrict__ ABp, const R* __restrict_
   }
 }
 
-// The same for launches whose threads are all on the chip at once (K <= 16, the rule stands at the
+// The same for launches whose blocks are all on the chip at once (K <= 16, the rule stands at the
 // launch): their time is the longest chain of one thread, not memory. So a P element, which
 // depends on no other, has a thread of its own (blockDim.x / K rows a block); partials load in
 // batches; the bias corrections are formed once a block, beside those loads; and the
 // lanes that added a Q row's partials (gq = 32) take its elements, the sums that normalise it
 // running over the lanes in the elements' order. A 20-iteration fit of 105 x 8,451, K=7 in
-// float32: 1.33 -> 1.24 ms. Larger launches want the form above: 20,000 x 100,000, K=6 took
+// float64: 1.33 -> 1.24 ms. Larger launches want the form above: 20,000 x 100,000, K=6 took
 // 3.82 ms with this one against 3.80, and 10,007 x 200,003, K=8 1.96 against 1.92.
 template <typename R, int KMAX>
 __device__ __forceinline__ void add_partials(double (&v)[KMAX], const R* __restrict__ src, int64_t stride, int K,
@@ -962,10 +962,11 @@ static int launch_update_from(const EmPlan& pl, const R* ABp, const R* Tp, int m
     return (rows <= 4096 && parts >= 32) || (rows < 16384 && parts >= 128) ? 32 : 1;
   };
   const int gp = lanes(pl.M, pl.n_split), gq = lanes(pl.N, pl.n_mblk);
-  // every thread of the launch on the chip at once (148 SMs, a constant): see the resident kernel
-  if (pl.K <= RESIDENT_MAX_K && gp == 1 && pl.M * pl.K + pl.N * gq <= 148 * RESIDENT_BLOCKS * RESIDENT_TPB) {
-    const unsigned pb = (unsigned)ceil_div(pl.M, RESIDENT_TPB / pl.K);
-    const unsigned blocks = pb + (unsigned)ceil_div(pl.N * gq, RESIDENT_TPB);
+  // every block of the launch on the chip at once (148 SMs, a constant): see the resident kernel
+  const int64_t resident_p = pl.K <= RESIDENT_MAX_K ? ceil_div(pl.M, RESIDENT_TPB / pl.K) : 0;
+  const int64_t resident = resident_p + ceil_div(pl.N * gq, RESIDENT_TPB);
+  if (pl.K <= RESIDENT_MAX_K && gp == 1 && resident <= 148 * RESIDENT_BLOCKS) {
+    const unsigned pb = (unsigned)resident_p, blocks = (unsigned)resident;
 #define LAUNCH(KM)                                                                                            \
   if constexpr (KM <= RESIDENT_MAX_K)                                                                         \
     em_update_resident_kernel<R, KM><<<blocks, RESIDENT_TPB, 0, st>>>(                                        \

@@ -54,3 +54,9 @@ def test_update_matches_the_oracle(cuda, N, M, K):
                           (dvQ, vQ, 1e-10)):
         assert np.abs(got.cpu().numpy() - ref).max() <= bar
     assert torch.equal(P32, Pd.float()) and torch.equal(Q32, Qd.float())
+
+
+# at the line between the two forms, 592 blocks and one more: 8 rows of K = 15 a block, 32 blocks of Q
+@pytest.mark.parametrize("M", [560 * 8, 560 * 8 + 1])
+def test_both_forms_at_their_line(cuda, M):
+    test_update_matches_the_oracle(cuda, 128, M, 15)

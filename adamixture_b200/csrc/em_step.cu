@@ -881,14 +881,15 @@ int em_plan(int64_t M, int64_t N, int K, int prec, EmPlan& pl) {
   // of the float32 pairs). Of 1 to 12 CTAs per SM (148, a constant, as above), the count whose
   // CTAs finish first, as many at a time as the registers allow (float64: 1). At N=105 x
   // M=8,451, K=7 in float64: 133 CTAs of 4 chunks in one round instead of 529 of one chunk in four.
-  // An iteration with PLAN_BLOCKS and with this rule: float64 K=10, 4,000 x 12,000 355 and 303 us,
-  // 4,000 x 30,000 (16 chunks and more: the rule does not apply) 772 both; from 4,096 samples the
-  // plan is left as it was. Float32 K=8, 5,000 x 30,000 527 and 402 us, 18,000 x 5,000 318 and 255;
+  // An iteration with PLAN_BLOCKS and with this rule: float64 K=10, 1,000 x 20,000 185 and 136 us,
+  // 2,504 x 20,003 359 and 321; but the float64 log-likelihood has the sweep's partition (its
+  // partials are the same), runs two CTAs per SM and loses from about 2,000 samples on (2,000 x
+  // 12,000 56 and 60 us, 2,504 x 20,003 95 and 117), so the line is at 2,048. Float32 K=8, 5,000 x 30,000 527 and 402 us, 18,000 x 5,000 318 and 255;
   // with K <= 4, whose chunks are short, 5,000 x 30,000 181 and 187, 16,000 x 30,000 536 and 517: no
   // gain to speak of above 2,048 samples.
   const bool mma64 = prec == ADX_F64 && K <= DMMA_MAX_K, pairs32 = prec == ADX_F32 && K <= f32s::MAX_K;
   const int64_t own_tiles = ceil_div(pl.n_stile, n_split);
-  const int64_t most = mma64 ? 4095 : K <= 4 ? 2048 : 19999;
+  const int64_t most = mma64 || K <= 4 ? 2048 : 19999;
   if ((mma64 || pairs32) && N <= most && own_tiles * (mb / CH) < 16) {
     const int64_t slots = mma64 ? 148 : 148 * f32s::ctas_per_sm(K), start = mma64 ? 4 : 1;
     auto rounds = [&]() { return ceil_div(n_split * n_mblk, slots) * own_tiles * (mb / CH + start); };

@@ -318,19 +318,25 @@ __device__ __forceinline__ void mma_f64_k8(double (&d)[4], double a0, double a1,
                : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
 }
 
+// Pair blocks of at most 10 column tiles, column tiles of a pair block, and the CTAs per SM that
+// their accumulators' registers allow: for the kernels and for the host's choice of splits.
+__host__ __device__ constexpr int pair_blocks(int K) { return (K * (K + 1) / 2 + 79) / 80; }
+__host__ __device__ constexpr int pair_tiles(int K) { return ((K * (K + 1) / 2 + pair_blocks(K) - 1) / pair_blocks(K) + 7) / 8; }
+__host__ __device__ constexpr int ctas_per_sm(int K) { return pair_tiles(K) <= 4 ? 4 : pair_tiles(K) <= 7 ? 3 : 2; }
+
 template <bool QSIDE, int K>
 struct Shape {
   static constexpr int KS = (K + 3) / 4;                       // h's k-steps of 4
   static constexpr int NTG = (K + 7) / 8;                      // gradient column tiles
   static constexpr int PAIRS = K * (K + 1) / 2;
-  static constexpr int NPB = (PAIRS + 79) / 80;                // pair blocks of at most 10 column tiles
-  static constexpr int NP = ((PAIRS + NPB - 1) / NPB + 7) / 8; // column tiles of a pair block
+  static constexpr int NPB = pair_blocks(K);
+  static constexpr int NP = pair_tiles(K);
   static constexpr int TPC = 8 * NP;
   static constexpr int COLS = TPC + 8 * NTG;                   // pairs, then the gradient's columns
   static constexpr int CS = COLS + 2;                          // = 2 mod 8: 16-byte fragment loads free of conflicts
   static constexpr int NT = QSIDE ? 2 : 1;
   static constexpr int FS = K <= 4 ? 4 : (K <= 12 ? 12 : 20);  // factor row stride: 4 or 12 mod 16, conflict-free
-  static constexpr int OCC = NP <= 4 ? 4 : NP <= 7 ? 3 : 2;     // CTAs per SM the registers allow
+  static constexpr int OCC = ctas_per_sm(K);
   static constexpr size_t SMEM = sizeof(double) * (CJ * FS + NT * CJ * CS);
 };
 
@@ -426,8 +432,10 @@ __global__ void __launch_bounds__(32 * MWARPS, Shape<QSIDE, K>::OCC) grad_hess_m
   const int64_t n_chunks = (n_red + CJ - 1) / CJ;
   const int64_t ch0 = (int64_t)split * a.chunks_per_split;
   const int64_t ch1 = min(n_chunks, ch0 + a.chunks_per_split);
-  // a chunk's genotypes and, where registers are left, its factor rows (contiguous; zeros past
-  // the axis) are loaded a chunk ahead of their use
+  // a chunk's genotypes and, where registers are left, its factor rows (contiguous; zeros past the
+  // axis) are loaded a chunk ahead of their use. With 6 or 7 column tiles (K = 9, 10, 13, 14) at 3
+  // CTAs per SM they spill: 7.6 ms on the P side at N=20,000 x M=50,000, K=10 where loading them at
+  // use takes 7.2
   constexpr bool AHEAD = NP <= 5 || NP >= 8;
   constexpr int FPT = (CJ * K + 32 * MWARPS - 1) / (32 * MWARPS);
   Codes next;
@@ -589,13 +597,6 @@ static int grad_hess_mma_launch(const gh::Args& a, int64_t blocks, cudaStream_t 
   return ADX_OK;
 }
 
-// Shape's constants that the host needs
-static int mma_pair_blocks(int K) { return (K * (K + 1) / 2 + 79) / 80; }
-static int mma_ctas_per_sm(int K) {
-  const int npb = mma_pair_blocks(K), np = ((K * (K + 1) / 2 + npb - 1) / npb + 7) / 8;
-  return np <= 4 ? 4 : np <= 7 ? 3 : 2;
-}
-
 template <bool QSIDE>
 static int grad_hess(const uint8_t* G, int64_t M, int64_t N, int K, const double* P, const double* Q,
                      double* XtX, double* Xtz, void* stream, const char* name) {
@@ -610,7 +611,7 @@ static int grad_hess(const uint8_t* G, int64_t M, int64_t N, int K, const double
   gh::Args a{G, P, Q, M, N, K, XtX, Xtz, 0, 0, 0};
   const int n_pairs = K * (K + 1) / 2;
   const bool mma = K <= 16;
-  a.n_pblk = mma ? mma_pair_blocks(K) : (n_pairs + gh::TP - 1) / gh::TP;
+  a.n_pblk = mma ? gh::pair_blocks(K) : (n_pairs + gh::TP - 1) / gh::TP;
   const int64_t tiles = ceil_div(n_rows, gh::TR);
   const int64_t n_chunks = ceil_div(n_red, gh::CJ);
   int64_t split;
@@ -619,7 +620,7 @@ static int grad_hess(const uint8_t* G, int64_t M, int64_t N, int K, const double
     // the one whose rounds finish first, counting chunks and about 3 chunks of prologue and
     // atomics per CTA (at M=50,000 SNPs, K=10 on the P side: 5 splits, 8.8 rounds, 7.2 ms; 3
     // splits, 5.3 rounds, 7.7 ms)
-    const int64_t slots = (int64_t)sm_count() * mma_ctas_per_sm(K);
+    const int64_t slots = (int64_t)sm_count() * gh::ctas_per_sm(K);
     int64_t best = -1;
     split = 1;
     for (int64_t round = 1; round <= 12; ++round) {

@@ -33,12 +33,11 @@ constexpr int LL_BLOCKS = 1776;
 constexpr float LL_SCALE = 2147483648.0f;  // 2^31: float32 P is held x LL_SCALE
 constexpr int LL_QUAD_EXP = 248;          // a quad's four factors carry (2^62)^4
 
-template <typename R, int KMAX>
-struct LlCfg {
-  static constexpr int SPT = (sizeof(R) == 4) ? (KMAX <= 16 ? 4 : (KMAX <= 32 ? 2 : 1))
-                                              : (KMAX <= 16 ? 2 : 1);
-  static constexpr int CH = 32;
-};
+// K > 16: samples per thread of loglik_kernel
+__host__ __device__ constexpr int ll_spt(bool f32, int kmax) { return f32 && kmax <= 32 ? 2 : 1; }
+// K <= 16: samples per sub-tile of the plan (float32: ll32's; float64: of the partial count that
+// the workspace query gives, the MMA form has its own tiles)
+constexpr int LL_SMALL_K = 16, LL_W32 = 1024, LL_W64 = 512;
 
 // Split x = m * 2^e with m in [0.5, 1): returns m, adds e to *e.
 __device__ __forceinline__ double renorm(double x, int& e) {
@@ -69,12 +68,11 @@ __device__ __forceinline__ void unpack_f32x2(unsigned long long v, float& lo, fl
 // vec: the host checked that N is a multiple of SPT and G is SPT-byte aligned, so a
 // thread's SPT bytes of a packed row are one aligned load.
 template <typename R, int KMAX>
-__global__ void __launch_bounds__(LL_TPB, KMAX <= 12 ? 3 : 1)
+__global__ void __launch_bounds__(LL_TPB, 1)
 loglik_kernel(const uint8_t* __restrict__ G, const R* __restrict__ P, const R* __restrict__ Q,
               int64_t M, int64_t N, int K, int64_t n_stile, int n_split, int n_mblk, int64_t mb,
               int vec, double* __restrict__ partial) {
-  using C = LlCfg<R, KMAX>;
-  constexpr int SPT = C::SPT, CH = C::CH;
+  constexpr int SPT = ll_spt(sizeof(R) == 4, KMAX), CH = 32;
   // float32 h of two samples at once with packed FMAs: P is kept duplicated {p, p}
   constexpr bool PAIRS = sizeof(R) == 4 && SPT % 2 == 0;
   __shared__ __align__(16) unsigned char ps_raw[CH * KMAX * (PAIRS ? 8 : sizeof(R))];
@@ -95,8 +93,7 @@ loglik_kernel(const uint8_t* __restrict__ G, const R* __restrict__ P, const R* _
     auto load_word = [&](int64_t row) -> uint32_t {
       const uint8_t* src = G + row * N + i0;
       if (vload) {
-        if constexpr (SPT == 4) return __ldg(reinterpret_cast<const unsigned int*>(src));
-        else if constexpr (SPT == 2) return (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(src));
+        if constexpr (SPT == 2) return (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(src));
         else return (uint32_t)__ldg(src);
       }
       uint32_t w = 0;
@@ -229,10 +226,10 @@ loglik_kernel(const uint8_t* __restrict__ G, const R* __restrict__ P, const R* _
 namespace ll32 {
 
 constexpr int TPB = 128;
-constexpr int C = 8;               // samples per thread: TPB * C = LL_TPB * 4, the same sub-tiles
+constexpr int C = 8;               // samples per thread
 constexpr int CH = 32;
-constexpr int MAX_K = 16;
-static_assert(TPB * C == LL_TPB * 4, "the plan's sub-tile width");
+constexpr int MAX_K = LL_SMALL_K;
+static_assert(TPB * C == LL_W32, "the plan's sub-tile width");
 using u64 = unsigned long long;
 
 __device__ __forceinline__ u64 mul2(u64 a, u64 b) {
@@ -380,18 +377,6 @@ struct LlPlan {
   int64_t mb;
 };
 
-template <typename R, int KMAX>
-static int spt_of() { return LlCfg<R, KMAX>::SPT; }
-
-#define ADX_LL_KMAX_SWITCH(kmax, MACRO)                                                \
-  switch (kmax) {                                                                      \
-    case 2: MACRO(2); break;   case 3: MACRO(3); break;   case 4: MACRO(4); break;     \
-    case 6: MACRO(6); break;   case 8: MACRO(8); break;   case 10: MACRO(10); break;   \
-    case 12: MACRO(12); break; case 16: MACRO(16); break; case 24: MACRO(24); break;   \
-    case 32: MACRO(32); break; case 48: MACRO(48); break; case 64: MACRO(64); break;   \
-    default: break;                                                                    \
-  }
-
 // Whether a thread's SPT bytes of a packed row can be one aligned load: N a multiple of
 // SPT (so every row starts SPT-aligned relative to G) and G itself SPT-byte aligned.
 static int ll_vec_loads(const uint8_t* G, int64_t N, int spt) {
@@ -402,14 +387,9 @@ static int ll_plan(int64_t M, int64_t N, int K, int prec, LlPlan& pl) {
   if (M <= 0 || N <= 0 || K < 1 || K > ADX_MAX_K) return ADX_ERR_ARG;
   if (prec != ADX_F64 && prec != ADX_F32 && prec != ADX_BF16 && prec != ADX_F16) return ADX_ERR_UNSUPPORTED;
   pl.kmax = pick_kmax(K);
-  int spt = 1;
-#define S64(KM) spt = spt_of<double, KM>()
-#define S32(KM) spt = spt_of<float, KM>()
-  if (prec == ADX_F64) { ADX_LL_KMAX_SWITCH(pl.kmax, S64) } else { ADX_LL_KMAX_SWITCH(pl.kmax, S32) }
-#undef S64
-#undef S32
-  pl.spt = spt;
-  pl.n_stile = ceil_div(N, (int64_t)LL_TPB * spt);
+  pl.spt = ll_spt(prec != ADX_F64, pl.kmax);
+  const int width = K > LL_SMALL_K ? LL_TPB * pl.spt : prec == ADX_F64 ? LL_W64 : LL_W32;
+  pl.n_stile = ceil_div(N, (int64_t)width);
   int64_t n_split = pl.n_stile < 8 ? pl.n_stile : 8;
   // at most LL_BLOCKS blocks (rounding the SNP blocks up to 32 rows only lowers the count),
   // so the grid never spills a few blocks into one more wave

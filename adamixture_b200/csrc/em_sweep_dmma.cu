@@ -154,10 +154,9 @@ __device__ __forceinline__ bool inside(const double (&x)[N], double lo) {
 // The genotype bytes of SNP rows g and g+8 of the chunk at jc for the thread's 8 samples from
 // s0. Rows past the matrix read its last row (those SNPs are masked as missing by the caller).
 // fetch: the aligned words that hold them, a chunk ahead of their use -- one 8-byte load where
-// every packed row is 8-byte aligned (VEC), else three words (byte loads through one thread
-// took the sweep from 27.9 to 37.2 ms at N=100,003 x M=50,000, K=10, and the log-likelihood from
-// 6.8 to 9.8 ms at N=50,003 x M=100,000, K=8: 28.3 and 7.0 ms with the words). Bytes past the
-// matrix are 0xFF.
+// every packed row is 8-byte aligned (VEC), else three words. Bytes past the matrix are 0xFF.
+// Unaligned rows, the sweep at N=100,003 x M=50,000, K=10: 37.2 ms by bytes, 28.3 by words; the
+// log-likelihood at N=50,003 x M=100,000, K=8: 9.8 and 7.0 ms.
 struct RowWords {
   uint32_t w0, w1, w2;
 };
@@ -599,7 +598,7 @@ __global__ void __launch_bounds__(TPB, Lay<TL>::OCC) em_sweep_dmma_kernel(Args a
 // h = clamp(P_j . Q_i, 1e-10, 1-1e-10). As in loglik_kernel, each thread multiplies the
 // per-entry factors h^g (1-h)^(2-g) (the product x*y of two values picked by the genotype's
 // two bits; 1 when missing) into one float64 running product, moves its exponent into an
-// integer after every 4 factors (>= 1e-80 together, so the product stays normal), and takes
+// integer after every 8 factors (>= 1e-160 together, so the product stays normal), and takes
 // one log at the end; per-CTA sums in a fixed order, per-CTA partials summed in block order.
 
 // shared memory of the log-likelihood: the Q and P tiles and the warp sums (doubles)
@@ -675,9 +674,9 @@ __global__ void __launch_bounds__(TPB, 2) loglik_dmma_kernel(Args a, const uint8
           if constexpr (KS & 1)
             mma_f64(hacc[nt], ph[KS - 1][0], ph[KS - 1][1], qt[qrow * QSTR + ((4 * (KS - 1) + t) ^ qsw(qrow))]);
         }
-        // one vote for the chunk's 16 values a thread: the clamps are rarely needed. They and a
-        // renormalisation per 4 factors instead of 8 took 8.08 ms where this takes 6.5 (N=50,000 x
-        // M=100,000, K=8); a vote per tile of 4 was slower than the clamps (8.8 ms)
+        // one vote for the chunk's 16 values a thread: the clamps are rarely needed. 6.5 ms at
+        // N=50,000 x M=100,000, K=8; with the clamps throughout and a renormalisation per 4 factors
+        // instead of 8, 8.08 ms; with a vote per tile of 4, 8.8 ms
         if (__all_sync(0xffffffffu, inside(hacc[0], LL_CLAMP) && inside(hacc[1], LL_CLAMP) &&
                                         inside(hacc[2], LL_CLAMP) && inside(hacc[3], LL_CLAMP))) {
 #pragma unroll

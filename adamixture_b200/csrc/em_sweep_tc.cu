@@ -52,10 +52,10 @@
 // H is there when they come back for it. T has two buffers and is read two steps later, when
 // abfree says that its last batch is done.
 //
-// Measured at N=200,000 x M=500,000, K=10: 75.1 ms (330 GB/s of algorithmic bytes, 106
-// TFLOP/s). One warp that loaded and issued everything took 113.9 ms: an MMA here (M=128, N=16)
-// runs for about 100 cycles beside the consumers, its issuer is held for as long, and each
-// wait of the issuer drained the pipe for some 450 cycles, 5,200 cycles a step in all.
+// N=200,000 x M=500,000, K=10: 75.1 ms (330 GB/s of algorithmic bytes, 106 TFLOP/s). An MMA of the
+// A/B and T batches (M=128, N=16) runs for about 100 cycles beside the consumers and holds its
+// issuer for as long, and a wait of the issuer drains the pipe for some 450 cycles: with one warp
+// that loads and issues everything a step takes 5,200 cycles instead of 3,450 (113.9 ms).
 // Every wait is bounded and also watches a shared abort word; on a timeout the kernel
 // records ADX_ERR_TIMEOUT in the status word, all warps leave their loops, it waits (bounded)
 // for its MMAs in flight, frees its TMEM and returns.
@@ -263,8 +263,8 @@ __global__ void q_to_tiles_kernel(const float* __restrict__ Q, int64_t N, int K,
 // chunks. Otherwise the 9 chunks from the 16-byte boundary at or below the row's first byte
 // (they cover the 128 samples at any offset); the consumers apply the offset, which is a
 // constant of the row within the tile (row_offset). A sample count that is not a multiple of
-// 16 is what real cohorts have: loading such rows byte by byte through one warp took 14.9 ms
-// where these chunks take the aligned shape's time (2.7 ms then, 1.9 ms now; N=10,007 x M=200,003, K=8).
+// 16 is what real cohorts have: N=10,007 x M=200,003, K=8 takes 1.9 ms, as the aligned shape
+// (loaded byte by byte through one warp: 15 ms).
 // Chunks that would leave the matrix (the last row or two) take byte loads; bytes past the
 // matrix are 0xFF (missing). Samples past N read the next row's bytes or 0xFF: their Q rows
 // are zero, so they add nothing to A and B, and their T is not written. Rows past the matrix

@@ -127,3 +127,46 @@ def test_several_launches(ops, N, M):
         once = product(G, f, F, M, out=torch.zeros_like(got)) if product is ops.rsvd_rows else \
             product(G, f, F, M, out=torch.zeros_like(got), accumulate=True)
         assert torch.equal(once[:, fine], got[:, fine])
+
+
+def test_products_in_a_row(ops):
+    # a product's kernels overlap at their ends: products that read what the one before wrote, over
+    # one workspace, without a pause and replayed from a graph, equal those run one at a time
+    N, M, L = 700, 5003, 20
+    G, f, X, gen = cohort(N, M, 9)
+    ws = ops.rsvd_workspace(G.device, M, N, L)
+    B0 = torch.randn((N, L), generator=gen, device="cuda")
+    B0[:, 3] *= 2.0 ** -24   # wide: the second level too
+    B0[5, 3] = 1.0
+    want, B = [], B0
+    for _ in range(6):
+        Y = ops.rsvd_rows(G, f, B, M)
+        torch.cuda.synchronize()
+        B = ops.rsvd_cols(G, f, Y, M) * 2.0 ** -12
+        torch.cuda.synchronize()
+        want.append(B)
+    Y, B = torch.empty((M, L), device="cuda"), B0.clone()
+
+    def chain():
+        out = []
+        for _ in range(6):
+            ops.rsvd_rows(G, f, B, M, out=Y, ws=ws)
+            ops.rsvd_cols(G, f, Y, M, out=B, ws=ws)
+            B.mul_(2.0 ** -12)
+            out.append(B.clone())
+        return out
+
+    assert all(torch.equal(a, b) for a, b in zip(chain(), want))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    B.copy_(B0)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        got = chain()
+    for _ in range(3):
+        B.copy_(B0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    ops.rsvd_check(ws)

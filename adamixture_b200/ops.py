@@ -488,9 +488,12 @@ def rsvd_workspace(device: torch.device, M: int, N: int, L: int) -> torch.Tensor
 
 def rsvd_check(ws: torch.Tensor) -> None:
     """Raise if a bounded wait of a product that used ``ws`` ran out since the last check (its
-    output is NaN then). Synchronises the current stream."""
+    output is NaN then). Synchronises the current stream; while that is being captured into a graph
+    it reads nothing, and the status stays for a later check."""
     import ctypes
 
+    if torch.cuda.is_current_stream_capturing():
+        return
     out = ctypes.c_int(0)
     call("adx_rsvd_status", ws.data_ptr(), ws.numel(), ctypes.addressof(out), _stream(ws.device))
     if out.value:

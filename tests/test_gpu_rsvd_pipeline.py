@@ -170,3 +170,22 @@ def test_products_in_a_row(ops):
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(got, want))
     ops.rsvd_check(ws)
+
+
+def test_frequencies_can_be_captured(ops):
+    # the status is not read while a graph is being captured
+    from adamixture_b200.model.warm_start import m_step_P
+
+    N, M, K = 200, 900, 5
+    G, f, X, gen = cohort(N, M, 10)
+    Q = torch.softmax(torch.randn((N, K), generator=gen, device="cuda"), 1).double()
+    want = m_step_P(G, Q, M)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        got = m_step_P(G, Q, M)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
